@@ -203,10 +203,10 @@ __global__ void end_step_kernel(StepState *ts, int nStage, double tLimit) {
   ts->tSimulation = t;
 }
 
-__global__ void dtmin_from_blocks(StepState *ts, const double *dtBlock, int nBlock) {
+__global__ void dtmin_from_blocks(StepState *ts, const double *dtBlock, int nPart) {
   __shared__ double w[32];
   double m = 1e300;
-  for (int b = threadIdx.x; b < nBlock; b += blockDim.x) m = fmin(m, dtBlock[b]);
+  for (int b = threadIdx.x; b < nPart; b += blockDim.x) m = fmin(m, dtBlock[b]);
   for (int off = 16; off > 0; off >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, off));
   if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = m;
   __syncthreads();
@@ -227,7 +227,8 @@ __global__ void copy_blocks(double *dst, const double *src, const int *blocks, i
 
 // -------------------------------------------------------------------------
 // TMA tensor maps: the state [block][var][k][j][i] as a 5D tensor with the
-// interior box and the three ghost-slab boxes of bx_stage3d.cuh
+// interior box and the three ghost-slab boxes of bx_stage3d.cuh, and those of
+// the tiles of bx_stage_unit.cuh
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -245,13 +246,17 @@ int encode_maps(void *base, bool fp32, int N, int nBlock, TmaMaps &m) {
   const cuuint64_t dims[5] = {(cuuint64_t)N, (cuuint64_t)N, (cuuint64_t)N, 8, (cuuint64_t)nBlock};
   const cuuint64_t strides[4] = {N * e, N * N * e, (cuuint64_t)N * N * N * e, 8ull * N * N * N * e};
   const cuuint32_t hx = (cuuint32_t)(16 / e);
-  const cuuint32_t boxes[4][5] = {{(cuuint32_t)N, (cuuint32_t)N, (cuuint32_t)N, 8, 1},
+  const cuuint32_t boxes[8][5] = {{(cuuint32_t)N, (cuuint32_t)N, (cuuint32_t)N, 8, 1},
                                   {hx, (cuuint32_t)N, (cuuint32_t)N, 8, 1},
                                   {(cuuint32_t)N, 2, (cuuint32_t)N, 8, 1},
-                                  {(cuuint32_t)N, (cuuint32_t)N, 2, 8, 1}};
+                                  {(cuuint32_t)N, (cuuint32_t)N, 2, 8, 1},
+                                  {(cuuint32_t)N, 4, 4, 8, 1},
+                                  {hx, 4, 4, 8, 1},
+                                  {(cuuint32_t)N, 2, 4, 8, 1},
+                                  {(cuuint32_t)N, 4, 2, 8, 1}};
   const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  CUtensorMap *out[4] = {&m.in, &m.xh, &m.yh, &m.zh};
-  for (int q = 0; q < 4; q++) {
+  CUtensorMap *out[8] = {&m.in, &m.xh, &m.yh, &m.zh, &m.uin, &m.uxh, &m.uyh, &m.uzh};
+  for (int q = 0; q < 8; q++) {
     CUresult r = encode(out[q], fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, base,
                         dims, strides, boxes[q], estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -351,6 +356,7 @@ StageArgs stage_args(int iStage, bool computeDt) {
   a.useDivb = g.sch.UseDivbSource; a.useHalfStep = g.sch.UseHalfStep; a.computeDt = computeDt;
   a.beta = g.sch.LimiterBeta; a.gamma = g.sch.Gamma; a.invGm1 = 1.0 / (g.sch.Gamma - 1.0);
   a.cfl = g.sch.Cfl;
+  a.dtFactor = a.useHalfStep ? (a.cfl * a.iStage) / a.nStage : a.cfl;
   a.fl = floors();
   set_reschange(a);
   a.old = g.A;
@@ -417,9 +423,9 @@ int tune_stage_impl() {
   TuneKnobInfo &k = tune_knob(kTuneStageGrid), &kf = tune_knob(kTuneStageVariant);
   if (!g.ready || !g.use3d || (k.tuned == 2 && kf.tuned == 2)) return BX_OK;
   StepState saved;
-  std::vector<double> dtSaved(g.nBlock);
+  std::vector<double> dtSaved((size_t)kDtParts * g.nBlock);
   CK(cudaMemcpyAsync(&saved, g.ts, sizeof(StepState), cudaMemcpyDeviceToHost, g.st));
-  CK(cudaMemcpyAsync(dtSaved.data(), g.dtBlock, sizeof(double) * g.nBlock, cudaMemcpyDeviceToHost, g.st));
+  CK(cudaMemcpyAsync(dtSaved.data(), g.dtBlock, sizeof(double) * dtSaved.size(), cudaMemcpyDeviceToHost, g.st));
   CK(cudaStreamSynchronize(g.st));
   const int v0 = k.value, f0 = kf.value;
   const bool fixG = k.tuned == 2, fixF = kf.tuned == 2 || g.shape != kShape888;  // variants: 8^3 only
@@ -492,7 +498,7 @@ int tune_stage_impl() {
     if (!fixF) kf.tuned = 1;
   }
   CK(cudaMemcpyAsync(g.ts, &saved, sizeof(StepState), cudaMemcpyHostToDevice, g.st));
-  CK(cudaMemcpyAsync(g.dtBlock, dtSaved.data(), sizeof(double) * g.nBlock, cudaMemcpyHostToDevice, g.st));
+  CK(cudaMemcpyAsync(g.dtBlock, dtSaved.data(), sizeof(double) * dtSaved.size(), cudaMemcpyHostToDevice, g.st));
   CK(cudaStreamSynchronize(g.st));
   if (g.graph) { cudaGraphExecDestroy(g.graph); g.graph = nullptr; }  // captured with the old shapes
   return r;
@@ -757,6 +763,7 @@ int bx_init(const bx_grid_desc *gd, const bx_scheme_params *sp) {
       }
     }
     q.volume = q.cellSize[0] * q.cellSize[1] * q.cellSize[2];
+    q.invVolume = 1.0 / q.volume;
     for (int d = 0; d < 3; d++) {
       q.area[d] = q.volume / q.cellSize[d];
       q.invHalf[d] = 0.5 / q.cellSize[d];
@@ -793,12 +800,12 @@ int bx_init(const bx_grid_desc *gd, const bx_scheme_params *sp) {
   CK(cudaMalloc(&g.order, sizeof(int) * g.nBlock));
   CK(cudaMalloc(&g.geom, sizeof(BlockGeom) * g.nBlock));
   CK(cudaMalloc(&g.ts, sizeof(StepState)));
-  CK(cudaMalloc(&g.dtBlock, sizeof(double) * g.nBlock));
+  CK(cudaMalloc(&g.dtBlock, sizeof(double) * kDtParts * g.nBlock));
   CK(cudaMemcpyAsync(g.nbr, g.nbrH.data(), sizeof(int) * 6 * g.nBlock, cudaMemcpyHostToDevice, g.st));
   CK(cudaMemcpyAsync(g.order, g.orderH.data(), sizeof(int) * g.nOwned, cudaMemcpyHostToDevice, g.st));
   if (g.nOwned < g.nBlock) CK(cudaMalloc(&g.haloIdx, sizeof(int) * g.nBlock));
   CK(cudaMemcpyAsync(g.geom, g.geomH.data(), sizeof(BlockGeom) * g.nBlock, cudaMemcpyHostToDevice, g.st));
-  CK(cudaMemsetAsync(g.dtBlock, 0, sizeof(double) * g.nBlock, g.st));
+  CK(cudaMemsetAsync(g.dtBlock, 0, sizeof(double) * kDtParts * g.nBlock, g.st));
   if (g.nSlab) {
     g.lcH.assign(gd->iLevelCoord_IB, gd->iLevelCoord_IB + 4 * g.nBlock);
     const size_t nFace = (size_t)g.nI * g.nI;
@@ -926,8 +933,11 @@ int bx_set_time(double tSimulation, int nStep) {
 int bx_get_block_dt(double *DtMax_B) {
   NEED_READY();
   if (!DtMax_B) return fail(BX_ERR_ARG, "null argument");
-  CK(cudaMemcpyAsync(DtMax_B, g.dtBlock, sizeof(double) * g.nBlock, cudaMemcpyDeviceToHost, g.st));
+  std::vector<double> parts((size_t)kDtParts * g.nBlock);
+  CK(cudaMemcpyAsync(parts.data(), g.dtBlock, sizeof(double) * parts.size(), cudaMemcpyDeviceToHost, g.st));
   CK(cudaStreamSynchronize(g.st));
+  for (int b = 0; b < g.nBlock; b++)
+    DtMax_B[b] = *std::min_element(parts.begin() + (size_t)kDtParts * b, parts.begin() + (size_t)kDtParts * (b + 1));
   return BX_OK;
 }
 
@@ -939,7 +949,9 @@ int bx_set_block_dt(const double *DtMax_B) {
     if (!(DtMax_B[b] > 0.0)) return fail(BX_ERR_ARG, "DtMax_B(%d) = %g", b + 1, DtMax_B[b]);
     m = std::min(m, DtMax_B[b]);
   }
-  CK(cudaMemcpyAsync(g.dtBlock, DtMax_B, sizeof(double) * g.nBlock, cudaMemcpyHostToDevice, g.st));
+  std::vector<double> parts((size_t)kDtParts * g.nBlock);
+  for (int b = 0; b < g.nBlock; b++) store_block_dt(parts.data(), b, DtMax_B[b]);
+  CK(cudaMemcpyAsync(g.dtBlock, parts.data(), sizeof(double) * parts.size(), cudaMemcpyHostToDevice, g.st));
   StepState s;
   CK(cudaMemcpyAsync(&s, g.ts, sizeof(s), cudaMemcpyDeviceToHost, g.st));
   CK(cudaStreamSynchronize(g.st));
@@ -1053,7 +1065,7 @@ int bx_set_global_timestep(double tLimit, double *Dt) {
   NEED_READY();
   // DtMax_B of the blocks whose calc_timestep ran through the per-block path
   if (g.scrDt) {
-    dtmin_from_blocks<<<1, 1024, 0, g.st>>>(g.ts, g.dtBlock, g.nBlock);
+    dtmin_from_blocks<<<1, 1024, 0, g.st>>>(g.ts, g.dtBlock, kDtParts * g.nBlock);
     CK(cudaGetLastError());
   }
   set_dt_kernel<<<1, 1, 0, g.st>>>(g.ts, tLimit, g.sch.UseDtFixed, g.sch.DtFixed, g.sch.Cfl);

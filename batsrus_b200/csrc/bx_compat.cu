@@ -141,7 +141,7 @@ __global__ void compat_timestep(CompatArgs a, int b) {
   if (threadIdx.x == 0) {
     double r = wmin[0];
     for (int w = 1; w < (int)(blockDim.x >> 5); w++) r = fmin(r, wmin[w]);
-    a.dtBlock[b] = r;
+    store_block_dt(a.dtBlock, b, r);
   }
 }
 

@@ -38,7 +38,15 @@ struct BlockGeom {
   double volume;
   double area[3];
   double invHalf[3];  // 0.5/CellSize (DxInvHalf of calc_divb_source)
+  double invVolume;   // 1/volume
 };
+
+// DtMax_B is kept in kDtParts parts per block (a unit of the 3D stage kernel
+// covers one quarter of an 8^3 block); DtMax_B is the smallest of them
+constexpr int kDtParts = 4;
+__host__ __device__ inline void store_block_dt(double *dt, int b, double m) {
+  for (int q = 0; q < kDtParts; q++) dt[(size_t)kDtParts * b + q] = m;
+}
 
 struct StageArgs {
   const void *in;          // gather source (double* or float*)
@@ -48,10 +56,11 @@ struct StageArgs {
   const int *order;        // processing order (Morton) of the blocks
   const BlockGeom *geom;   // [nBlock]
   StepState *ts;
-  double *dtBlock;         // optional DtMax_B per block
+  double *dtBlock;         // optional DtMax_B, kDtParts per block
   int nBlock;
   int iStage, nStage, nOrder, limiter, useDivb, useHalfStep, computeDt;
   double beta, gamma, invGm1, cfl;
+  double dtFactor = 0.0;   // the stage's part of the time step: cfl, or cfl iStage/nStage (half step scheme)
   // residual mode of the 3D kernel (get_residual of the implicit scheme):
   // the input holds total energy in the pressure slot, the output is the
   // increment dtScale*DtMax_CB*(S + dF/V) of the implicit variables, with
@@ -96,7 +105,7 @@ struct CompatArgs {
   double *left[3], *right[3], *flux[3];  // face scratch of one block
   double *source;          // Source_VC scratch (9 per cell)
   double *dtCell;          // DtMax_CB of the block (nCell)
-  double *dtBlock;         // DtMax_B
+  double *dtBlock;         // DtMax_B, kDtParts per block
   int iStage, nStage, nOrder, limiter, useDivb, useHalfStep;
   double beta, gamma, invGm1, cfl;
   Floors fl;
@@ -113,9 +122,11 @@ cudaError_t launch_stage_fp32(int shape, int flux, int kind, const StageArgs &a,
 cudaError_t launch_compat(int shape, int flux, int phase, int iBlock, const CompatArgs &a,
                           cudaStream_t st);
 // persistent TMA-staged kernel of 3D shapes (bx_stage3d.cu): tensor maps of
-// the stage input for the interior box and the x, y, z ghost slabs
+// the stage input for the interior box and the x, y, z ghost slabs of a
+// block, and those of a tile of 4 x 4 rows (bx_stage_unit.cuh)
 struct alignas(64) TmaMaps {
   CUtensorMap in, xh, yh, zh;
+  CUtensorMap uin, uxh, uyh, uzh;
 };
 enum { kKindFp64 = 0, kKindFp32In64 = 1, kKindFp32In32 = 2 };
 cudaError_t launch_stage3d(int shape, int flux, int kind, const TmaMaps &maps, const StageArgs &a, int nSM,

@@ -22,12 +22,12 @@ enum { kLimMinmod = 0, kLimMc = 1, kLimMc3 = 2 };
 template <typename R>
 __device__ __forceinline__ R sign25(R x) { return copysign(R(0.25), x); }
 
-// Division, reciprocal and square root of the face arithmetic: IEEE in
-// double (the FP64 mode matches the CPU oracle to rounding); in float the
+// Division, reciprocal and square root of the face arithmetic.  In float the
 // hardware approximations, div.approx.f32 (__fdividef), rcp.approx.ftz.f32
 // and sqrt.approx.ftz.f32 (PTX ISA), a few ulp, far inside the FP32-bulk
 // mode's bound on the error against FP64 (the operands are positive normal
-// numbers: densities, pressures, wave-speed sums)
+// numbers: densities, pressures, wave-speed sums).  In double the IEEE
+// operations; the explicit 3D kernel uses the branch-free forms below.
 __device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double frcp(double a) { return 1.0 / a; }
@@ -42,6 +42,47 @@ __device__ __forceinline__ float fsqrt(float a) {
   asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
   return r;
 }
+
+// Branch-free double reciprocal, quotient and square roots: the hardware
+// seed rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64 (PTX ISA, about 20 bits),
+// then one third-order step of the binomial series: with e = 1 - a y,
+// 1/a = y (1 + e + e^2 + ...); with e = 1 - a y^2,
+// 1/sqrt(a) = y (1 + e/2 + 3 e^2/8 + ...).  The neglected term is of the order of
+// e^3 = 2^-60, so the result is within one unit in the last place; the
+// quotient is corrected once with its remainder.  Normal operands; a zero
+// operand gives NaN where the IEEE operation gives infinity (sqrt_nb: the
+// callers add a tiny number that keeps the argument from zero).
+__device__ __forceinline__ double rcp_nb(double a) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-a, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ float rcp_nb(float a) { return frcp(a); }
+__device__ __forceinline__ double div_nb(double a, double b) {
+  const double y = rcp_nb(b), q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+__device__ __forceinline__ float div_nb(float a, float b) { return __fdividef(a, b); }
+// num / sqrt(a): with num = a the square root of a
+__device__ __forceinline__ double over_sqrt_nb(double num, double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-(a * y), y, 1.0), s = num * y;
+  return fma(s * e, fma(e, 0.375, 0.5), s);
+}
+__device__ __forceinline__ double sqrt_nb(double a) { return over_sqrt_nb(a, a); }
+__device__ __forceinline__ float sqrt_nb(float a) { return fsqrt(a); }
+__device__ __forceinline__ double sqrt0_nb(double a) { return sqrt_nb(a + 1e-290); }
+__device__ __forceinline__ float sqrt0_nb(float a) { return fsqrt(a); }
+
+// the smaller and the larger of two numbers: a comparison and a select in
+// double (fmin and fmax spend more instructions on NaN, which a face state
+// carries into its flux either way)
+__device__ __forceinline__ double lo2(double a, double b) { return a < b ? a : b; }
+__device__ __forceinline__ double hi2(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ float lo2(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ float hi2(float a, float b) { return fmaxf(a, b); }
 
 // limit_pressure (src/ModEnergy.f90:388-420) for the single ion fluid: the
 // pressure floor pMin, then the temperature floor NumDens*TMin with
@@ -78,26 +119,57 @@ __device__ __forceinline__ void limited_face(int lim, R beta, R q0, R q1, R q2, 
   right = q2 - dR;
 }
 
-// limited_face with the limiter fixed at compile time (same arithmetic)
-template <int LIM, typename R>
-__device__ __forceinline__ void limited_face_t(R beta, R q0, R q1, R q2, R q3, R &left, R &right) {
-  const R a = q1 - q0, b = q2 - q1, c = q3 - q2;
-  const R sab = sign25(a) + sign25(b);
-  const R sbc = sign25(b) + sign25(c);
-  R dL, dR;
+// limited_face with the limiter fixed at compile time (the same results).
+// float: as written there.
+template <int LIM>
+__device__ __forceinline__ void limited_face_t(float beta, float q0, float q1, float q2, float q3, float &left,
+                                               float &right) {
+  const float a = q1 - q0, b = q2 - q1, c = q3 - q2;
+  const float sab = sign25(a) + sign25(b);
+  const float sbc = sign25(b) + sign25(c);
+  float dL, dR;
   if (LIM == kLimMinmod) {
     dL = sab * fmin(fabs(a), fabs(b));
     dR = sbc * fmin(fabs(b), fabs(c));
   } else if (LIM == kLimMc) {
-    dL = sab * fmin(fmin(beta * fabs(a), beta * fabs(b)), R(0.5) * fabs(a + b));
-    dR = sbc * fmin(fmin(beta * fabs(b), beta * fabs(c)), R(0.5) * fabs(b + c));
+    dL = sab * fmin(fmin(beta * fabs(a), beta * fabs(b)), 0.5f * fabs(a + b));
+    dR = sbc * fmin(fmin(beta * fabs(b), beta * fabs(c)), 0.5f * fabs(b + c));
   } else {
-    const R cThird = R(1) / R(3);
+    const float cThird = 1.0f / 3.0f;
     dL = sab * fmin(fmin(beta * fabs(a), beta * fabs(b)), cThird * fabs(a + 2 * b));
     dR = sbc * fmin(fmin(beta * fabs(b), beta * fabs(c)), cThird * fabs(2 * b + c));
   }
   left = q1 + dL;
   right = q2 - dR;
+}
+
+// double: the slopes with the sign of b taken out (a and c flipped where b
+// is negative), so that opposite signs show as a negative a or c: then the
+// smaller of a and |b| is negative and the slope is cut to zero.  The factors
+// 1/2 of the signs' mean go into the constants (exact), min(beta a, beta b)
+// is beta min(a, b) (rounding is monotonic): the same numbers as above with
+// 15 double operations instead of 18 and two comparisons fewer
+__device__ __forceinline__ double flip_sign(double x, double s) {
+  return __hiloint2double(__double2hiint(x) ^ (__double2hiint(s) & 0x80000000), __double2loint(x));
+}
+// m >= 0 where a >= 0: m with the sign of s, or zero where a is negative
+__device__ __forceinline__ double sign_or_zero(double m, double a, double s) {
+  const int keep = ~(__double2hiint(a) >> 31);
+  return __hiloint2double((__double2hiint(m) ^ (__double2hiint(s) & 0x80000000)) & keep, __double2loint(m) & keep);
+}
+template <int LIM>
+__device__ __forceinline__ double limited_slope(double halfBeta, double a, double b) {
+  const double m = lo2(a, b);
+  if (LIM == kLimMinmod) return 0.5 * m;
+  if (LIM == kLimMc) return lo2(halfBeta * m, 0.25 * (a + b));
+  return lo2(halfBeta * m, (0.5 * (1.0 / 3.0)) * fma(2.0, b, a));
+}
+template <int LIM>
+__device__ __forceinline__ void limited_face_t(double beta, double q0, double q1, double q2, double q3, double &left,
+                                               double &right) {
+  const double b = q2 - q1, a = flip_sign(q1 - q0, b), c = flip_sign(q3 - q2, b), h = 0.5 * beta, ab = fabs(b);
+  left = q1 + sign_or_zero(limited_slope<LIM>(h, a, ab), a, b);
+  right = q2 - sign_or_zero(limited_slope<LIM>(h, c, ab), c, b);
 }
 
 // limited_face_t with separate Beta for the two cells of the face: betaL for
@@ -402,7 +474,7 @@ __device__ __forceinline__ bool numerical_flux(R (&L)[8], R (&Rt)[8], R gamma, R
 }
 
 // ---------------------------------------------------------------------------
-// Register-light flux for the fused 3D kernel.  Same mathematics as
+// Register-light flux of the 3D kernels.  Same mathematics as
 // numerical_flux (get_numerical_flux with lax_friedrichs_flux /
 // harten_lax_vanleer_flux and Linde's fix), written component by component
 // so that only the two face states and a few scalars are live, with one
@@ -499,6 +571,316 @@ __device__ __forceinline__ R flux_lean(R (&L)[8], R (&Rt)[8], R gamma, R invGm1,
     out[7 * ostride] = area * f;
   }
   return area * cmax;
+}
+
+// ---------------------------------------------------------------------------
+// Rusanov and Linde flux of the explicit 3D kernel, in the face's own frame: states
+// (rho, u_n, u_t1, u_t2, b_n, b_t1, b_t2, p) with t1, t2 = n + 1, n + 2
+// (cyclic).  Same mathematics as numerical_flux (get_numerical_flux with
+// lax_friedrichs_flux / harten_lax_vanleer_flux and Linde's fix), agreeing
+// with it to rounding, with fewer operations:
+//  * the terms that cancel are left out: the normal induction flux
+//    u_n b_n - u_n b_n of each side, and after Linde's fix the jump of b_n;
+//  * the averaged state enters as sums, its factors 1/2 in the constants;
+//  * in double the fast speed c = sqrt((G + sqrt(G^2 - 4 gamma p b_n^2)) / 2 rho),
+//    G = gamma p + B^2, takes two reciprocal square roots and no reciprocal;
+//    in float G^2 would leave the range for SI units, so the sums are
+//    divided by the density first (get_mhd_speed's form);
+//  * the area multiplies the three HLL weights instead of the eight fluxes.
+// Measured with the limiter's and the update's counterparts: see
+// bx_stage_unit.cuh.
+
+// fast magnetosonic speed; gp = gamma p, b2 = B^2, bn4 = 4 b_n^2, rho2 = 2 rho
+__device__ __forceinline__ double fast_speed(double gp, double b2, double bn4, double rho2) {
+  const double g = gp + b2;
+  const double m = g + sqrt_nb(hi2(1e-280, fma(g, g, -(gp * bn4))));
+  return over_sqrt_nb(m, fma(m, rho2, 1e-290));
+}
+__device__ __forceinline__ float fast_speed(float gp, float b2, float bn4, float rho2) {
+  const float i = 2.0f * frcp(rho2), s = gp * i, f = (gp + b2) * i;
+  return fsqrt(0.5f * (f + fsqrt(fmaxf(0.0f, f * f - s * (bn4 * i)))));
+}
+
+// The 8 fluxes times area go to out(q, flux), q in the frame's order with the
+// energy flux last; returns Vdt.
+template <int FLUX, typename R, class Out>
+__device__ __forceinline__ R flux_frame(const R (&L)[8], const R (&Rt)[8], R gamma, R invGm1, R area, const Out &out) {
+  const R rL = L[0], rR = Rt[0], unL = L[1], unR = Rt[1], pL = L[7], pR = Rt[7];
+  // UseLindeFix (src/ModFaceFlux.f90:2302-2320): both sides get the mean b_n
+  const R dBn = R(0.5) * (Rt[4] - L[4]);
+  const R bnM = L[4] + dBn;
+  const R bnL = FLUX != kFluxRusanov ? bnM : L[4], bnR = FLUX != kFluxRusanov ? bnM : Rt[4];
+  const R B2L = bnL * bnL + L[5] * L[5] + L[6] * L[6];
+  const R B2R = bnR * bnR + Rt[5] * Rt[5] + Rt[6] * Rt[6];
+  const R bn4 = R(4) * (bnM * bnM);
+  // Cmax of the averaged state, and the weights of the two sides
+  const R unA = R(0.5) * (unL + unR), t1 = L[5] + Rt[5], t2 = L[6] + Rt[6];
+  const R fastA = fast_speed((R(0.5) * gamma) * (pL + pR), R(0.25) * (bn4 + (t1 * t1 + t2 * t2)), bn4, rL + rR);
+  const R cmax = fabs(unA) + fastA;
+  R aL, aR, ad;
+  if (FLUX == kFluxRusanov) {
+    aL = aR = R(0.5) * area;
+    ad = aL * cmax;
+  } else {
+    const R fastL = fast_speed(gamma * pL, B2L, bn4, R(2) * rL);
+    const R fastR = fast_speed(gamma * pR, B2R, bn4, R(2) * rR);
+    const R cl = lo2(R(0), lo2(unL - fastL, unA - fastA));
+    const R cr = hi2(R(0), hi2(unR + fastR, unA + fastA));
+    const R wL = div_nb(cr, cr - cl), wR = R(1) - wL;
+    aL = wL * area;
+    aR = wR * area;
+    ad = cr * aR;
+  }
+  // mass and momentum
+  const R mL = rL * unL, mR = rR * unR;
+  const R ptL = pL + R(0.5) * B2L, ptR = pR + R(0.5) * B2R;
+  out(0, aR * mR + aL * mL - ad * (rR - rL));
+  out(1, aR * (mR * unR - bnR * bnR + ptR) + aL * (mL * unL - bnL * bnL + ptL) - ad * (mR - mL));
+  R poyL = R(0), poyR = R(0);  // Poynting flux by the induction fluxes
+  R u2L = unL * unL, u2R = unR * unR;
+#pragma unroll
+  for (int c = 2; c < 4; c++) {
+    const R uL = L[c], uR = Rt[c], bL = L[c + 3], bR = Rt[c + 3];
+    out(c, aR * (mR * uR - bnR * bR) + aL * (mL * uL - bnL * bL) - ad * (rR * uR - rL * uL));
+    const R fL = unL * bL - uL * bnL, fR = unR * bR - uR * bnR;
+    out(c + 3, aR * fR + aL * fL - ad * (bR - bL));
+    poyL = poyL + fL * bL;
+    poyR = poyR + fR * bR;
+    u2L = u2L + uL * uL;
+    u2R = u2R + uR * uR;
+  }
+  const R vdt = cmax * area;
+  // the jump of b_n: Lax-Friedrichs diffusion (:2403-2418), or the Rusanov dissipation
+  out(4, FLUX != kFluxRusanov ? -(vdt * dBn) : -(ad * (bnR - bnL)));
+  const R eL = invGm1 * pL + R(0.5) * (rL * u2L), eR = invGm1 * pR + R(0.5) * (rR * u2R);
+  R fe = aR * (unR * (eR + pR) + poyR) + aL * (unL * (eL + pL) + poyL) -
+         ad * ((eR - eL) + R(0.5) * (B2R - B2L));
+  if (FLUX != kFluxRusanov) fe = fe - vdt * (bnM * dBn);
+  out(7, fe);
+  return vdt;
+}
+
+// hlld_flux with Linde's fix (get_numerical_flux, src/ModFaceFlux.f90:2130-2473,
+// 2826-3160) in the face's frame.  The formulas of the two sides of the
+// contact are mirror images, so the side that the contact moves away from
+// (near, sg = 1 for the left one) and the other (far) are selected once and
+// one copy of the code serves both: no divergence between faces with
+// opposite Un, half the instructions in the cache.  False where the
+// reference stops (negative density ratio).
+template <typename R, class Out>
+__device__ __forceinline__ bool hlld_frame(const R (&L)[8], const R (&Rt)[8], R gamma, R invGm1, R area, R &vdt,
+                                           const Out &out) {
+  const R cTiny = R(1.0e-6);
+  const R dBn = R(0.5) * (Rt[4] - L[4]), Bn = L[4] + dBn, Bn2 = Bn * Bn;
+  const R b2L = L[5] * L[5] + L[6] * L[6], b2R = Rt[5] * Rt[5] + Rt[6] * Rt[6];
+  const R cL = fast_speed(gamma * L[7], Bn2 + b2L, R(4) * Bn2, R(2) * L[0]);
+  const R cR = fast_speed(gamma * Rt[7], Bn2 + b2R, R(4) * Bn2, R(2) * Rt[0]);
+  const R sL = lo2(L[1] - cL, Rt[1] - cR), sR = hi2(L[1] + cL, Rt[1] + cR);
+  const R cmax = hi2(sR, -sL);
+  vdt = cmax * area;
+  const R ptL = L[7] + R(0.5) * (Bn2 + b2L), ptR = Rt[7] + R(0.5) * (Bn2 + b2R);
+  const R DsL = sL - L[1], DsR = sR - Rt[1], DrL = DsL * L[0], DrR = DsR * Rt[0];
+  const R inv = rcp_nb(DrR - DrL);
+  const R Un = (DrR * Rt[1] - DrL * L[1] - ptR + ptL) * inv;
+  const R pt12 = (DrR * ptL - DrL * ptR + DrR * DrL * (Rt[1] - L[1])) * inv;
+  const bool super = sL >= R(0) || sR <= R(0);
+  const bool left = super ? sL >= R(0) : Un >= R(0);
+  // near and far states: rho, u_n, u_t1, u_t2, b_t1, b_t2, p
+  const R rN = left ? L[0] : Rt[0], uN = left ? L[1] : Rt[1], v1N = left ? L[2] : Rt[2], v2N = left ? L[3] : Rt[3];
+  const R b1N = left ? L[5] : Rt[5], b2N = left ? L[6] : Rt[6], pN = left ? L[7] : Rt[7];
+  const R ptN = left ? ptL : ptR;
+  const R eN = invGm1 * pN + (ptN - pN) + R(0.5) * (rN * (uN * uN + v1N * v1N + v2N * v2N));
+  const R ubN = uN * Bn + v1N * b1N + v2N * b2N;
+  R rho, un, v1, v2, b1, b2, pt, e, ub;
+  bool ok = true;
+  if (super) {
+    // the flow is faster than every wave: the near state's own flux
+    rho = rN; un = uN; v1 = v1N; v2 = v2N; b1 = b1N; b2 = b2N; pt = ptN; e = eN; ub = ubN;
+  } else {
+    const R sg = left ? R(1) : R(-1), sN = left ? sL : sR, DsN = left ? DsL : DsR, DrN = left ? DrL : DrR;
+    un = Un;
+    pt = pt12;
+    // one outer star state: density factor, tangential velocity and field
+    auto star = [&](R Ds, R Dr, R gap, R u, R w1, R w2, R c1, R c2, R &o1, R &o2, R &p1, R &p2) {
+      const R den = Dr * gap - Bn2;
+      const bool plain = den < cTiny;
+      const R t = rcp_nb(plain ? R(1) : den);
+      const R fu = plain ? R(0) : Bn * (Un - u) * t, fb = plain ? R(1) : (Dr * Ds - Bn2) * t;
+      o1 = w1 - fu * c1;
+      o2 = w2 - fu * c2;
+      p1 = c1 * fb;
+      p2 = c2 * fb;
+    };
+    const R gapN = sN - Un, ig = rcp_nb(gapN);
+    R v1s, v2s, b1s, b2s;
+    star(DsN, DrN, gapN, uN, v1N, v2N, b1N, b2N, v1s, v2s, b1s, b2s);
+    rho = DrN * ig;
+    const R ubs = Un * Bn + v1s * b1s + v2s * b2s;
+    e = (DsN * eN - ptN * uN + pt12 * Un + Bn * (ubN - ubs)) * ig;
+    const R sqN = sqrt_nb(rho), aBn = fabs(Bn);
+    if (sg * Un - div_nb(aBn, sqN) >= R(0)) {
+      v1 = v1s; v2 = v2s; b1 = b1s; b2 = b2s; ub = ubs;
+    } else {
+      // between the Alfven waves
+      const R uF = left ? Rt[1] : L[1], v1F = left ? Rt[2] : L[2], v2F = left ? Rt[3] : L[3];
+      const R b1F = left ? Rt[5] : L[5], b2F = left ? Rt[6] : L[6];
+      const R sF = left ? sR : sL, DsF = left ? DsR : DsL, DrF = left ? DrR : DrL, gapF = sF - Un;
+      const R ratio = div_nb(DrF, gapF);
+      if (ratio < R(0)) ok = false;
+      const R sqF = sqrt0_nb(fabs(ratio));
+      R v1f, v2f, b1f, b2f;
+      star(DsF, DrF, gapF, uF, v1F, v2F, b1F, b2F, v1f, v2f, b1f, b2f);
+      const R t = rcp_nb(sqN + sqF), sB = copysign(R(1), Bn), ss = sg * sB, sNF = sqN * sqF * ss;
+      v1 = (sqN * v1s + sqF * v1f + (b1f - b1s) * ss) * t;
+      v2 = (sqN * v2s + sqF * v2f + (b2f - b2s) * ss) * t;
+      b1 = (sqN * b1f + sqF * b1s + (v1f - v1s) * sNF) * t;
+      b2 = (sqN * b2f + sqF * b2s + (v2f - v2s) * sNF) * t;
+      ub = Un * Bn + v1 * b1 + v2 * b2;
+      e = e - ss * (sqN * (ubs - ub));
+    }
+  }
+  const R m = area * (rho * un), aB = area * Bn, au = area * un;
+  out(0, m);
+  out(1, m * un - aB * Bn + area * pt);
+  out(2, m * v1 - aB * b1);
+  out(3, m * v2 - aB * b2);
+  out(4, -(vdt * dBn));
+  out(5, au * b1 - aB * v1);
+  out(6, au * b2 - aB * v2);
+  out(7, au * (e + pt) - aB * ub - vdt * (Bn * dBn));
+  return ok;
+}
+
+// ---------------------------------------------------------------------------
+// The same in float on packed pairs (add, mul and fma .f32x2 of sm_100: two
+// single-precision operations per instruction).  A pair holds the left and
+// the right state of a variable, so the whole flux but for the averaged
+// state and the weights runs packed.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ F2 f2(float x) { return f2(x, x); }
+__device__ __forceinline__ void f2_get(F2 a, float &x, float &y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+  F2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+// limited_face_t in float as the pair (left, right): with a, b, c the
+// differences of the stencil, (q0, q3) - (q1, q2) = (-a, c) carries both outer
+// differences; the same numbers as limited_face_t
+template <int LIM>
+__device__ __forceinline__ F2 limited_pair(float beta, float q0, float q1, float q2, float q3) {
+  const F2 mid = f2(q1, q2), d = f2(q0, q3) - mid;
+  const float b = q2 - q1;
+  float dx, dy, mL, mR;
+  f2_get(d, dx, dy);
+  if (LIM == kLimMinmod) {
+    mL = fminf(fabsf(dx), fabsf(b));
+    mR = fminf(fabsf(dy), fabsf(b));
+  } else {
+    const float k = LIM == kLimMc ? 1.0f : 2.0f;
+    const F2 t = fma2(f2(b), f2(-k, k), d) * f2(LIM == kLimMc ? 0.5f : 1.0f / 3.0f);
+    const float bb = fabsf(beta * b);
+    float tx, ty, ex, ey;
+    f2_get(t, tx, ty);
+    f2_get(d * f2(beta), ex, ey);
+    mL = fminf(fminf(fabsf(ex), bb), fabsf(tx));
+    mR = fminf(fminf(fabsf(ey), bb), fabsf(ty));
+  }
+  const F2 s = f2(sign25(-dx), sign25(-dy)) + f2(sign25(b), sign25(-b));
+  return fma2(s, f2(mL, mR), mid);
+}
+
+// flux_frame on pairs
+template <int FLUX, class Out>
+__device__ __forceinline__ float flux_pair(const F2 (&X)[8], float gamma, float invGm1, float area, const Out &out) {
+  float rL, rR, unL, unR, pL, pR, bL, bR, x, y;
+  f2_get(X[0], rL, rR);
+  f2_get(X[1], unL, unR);
+  f2_get(X[4], bL, bR);
+  f2_get(X[7], pL, pR);
+  const float dBn = 0.5f * (bR - bL), bnM = bL + dBn;
+  // the two sides' normal field and its negative
+  const F2 BN = FLUX != kFluxRusanov ? f2(bnM) : X[4];
+  const F2 nBN = FLUX != kFluxRusanov ? f2(-bnM) : X[4] * f2(-1.0f);
+  const F2 B2 = fma2(BN, BN, fma2(X[6], X[6], X[5] * X[5]));
+  const float bn4 = 4.0f * (bnM * bnM), unA = 0.5f * (unL + unR);
+  float t1, t2;
+  f2_get(X[5], x, y);
+  t1 = x + y;
+  f2_get(X[6], x, y);
+  t2 = x + y;
+  const float fastA = fast_speed((0.5f * gamma) * (pL + pR), 0.25f * (bn4 + (t1 * t1 + t2 * t2)), bn4, rL + rR);
+  const float cmax = fabsf(unA) + fastA;
+  float aL, aR, ad;
+  if (FLUX == kFluxRusanov) {
+    aL = aR = 0.5f * area;
+    ad = aL * cmax;
+  } else {
+    // both sides' fast speeds (fast_speed)
+    const F2 i = f2(frcp(rL), frcp(rR)), gp = X[7] * f2(gamma), f = (gp + B2) * i;
+    f2_get(fma2(gp * i, f2(-bn4) * i, f * f), x, y);
+    f2_get((f + f2(fsqrt(fmaxf(0.0f, x)), fsqrt(fmaxf(0.0f, y)))) * f2(0.5f), x, y);
+    const float cl = fminf(0.0f, fminf(unL - fsqrt(x), unA - fastA));
+    const float cr = fmaxf(0.0f, fmaxf(unR + fsqrt(y), unA + fastA));
+    const float wL = div_nb(cr, cr - cl);
+    aL = wL * area;
+    aR = (1.0f - wL) * area;
+    ad = cr * aR;
+  }
+  const F2 M = X[0] * X[1];
+  auto put = [&](int q, F2 f, F2 u) {  // fluxes f, conserved variables u of the two sides
+    float fx, fy, ux, uy;
+    f2_get(f, fx, fy);
+    f2_get(u, ux, uy);
+    out(q, aR * fy + aL * fx - ad * (uy - ux));
+  };
+  put(0, M, X[0]);
+  put(1, fma2(M, X[1], fma2(nBN, BN, fma2(B2, f2(0.5f), X[7]))), M);
+  F2 poy, u2 = X[1] * X[1];
+#pragma unroll
+  for (int c = 2; c < 4; c++) {
+    put(c, fma2(M, X[c], nBN * X[c + 3]), X[0] * X[c]);
+    const F2 f = fma2(X[1], X[c + 3], nBN * X[c]);
+    put(c + 3, f, X[c + 3]);
+    poy = c == 2 ? f * X[5] : fma2(f, X[6], poy);
+    u2 = fma2(X[c], X[c], u2);
+  }
+  const float vdt = cmax * area;
+  out(4, FLUX != kFluxRusanov ? -(vdt * dBn) : -(ad * (bR - bL)));
+  const F2 e = fma2(X[0] * u2, f2(0.5f), X[7] * f2(invGm1));
+  const F2 fe = fma2(X[1], e + X[7], poy), eT = fma2(B2, f2(0.5f), e);
+  float fx, fy, ex, ey;
+  f2_get(fe, fx, fy);
+  f2_get(eT, ex, ey);
+  float o = aR * fy + aL * fx - ad * (ey - ex);
+  if (FLUX != kFluxRusanov) o = o - vdt * (bnM * dBn);
+  out(7, o);
+  return vdt;
 }
 
 // ---------------------------------------------------------------------------

@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(S::NTHREAD, 1) stage_kernel(StageArgs a) {
     if (threadIdx.x == 0) {
       double m = wmin[0];
       for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmin(m, wmin[w]);
-      if (a.dtBlock) a.dtBlock[b] = m;
+      if (a.dtBlock) store_block_dt(a.dtBlock, b, m);
       atomicMin(&a.ts->DtMinBits, dbits(m));
     }
   }

@@ -151,6 +151,14 @@ __device__ __forceinline__ int face_id(int i, int j, int k) {
   return i + N * (j + N * k);
 }
 
+// 1/rho of the conversion: IEEE in double; in float one Newton step on the
+// hardware approximation (IEEE rounding but for rare last bits), branch-free
+__device__ __forceinline__ double cell_rcp(double x) { return 1.0 / x; }
+__device__ __forceinline__ float cell_rcp(float x) {
+  const float y = frcp(x);
+  return fmaf(fmaf(-x, y, 1.0f), y, y);
+}
+
 // the ten face slots of one face from its left and right primitive states:
 // fluxes times area (0..7), Vdt (8), BnL + BnR (9); false where hlld_flux
 // stops.  cbL, cbR, cuL, cuR: the normal field and normal velocity of the
@@ -170,16 +178,38 @@ __device__ __forceinline__ bool face_slots(Real (&L)[8], Real (&R)[8], Real gamm
     return true;
   }
   out[9 * stride] = L[kBx + D] + R[kBx + D];
-  if (FLUX == kFluxHlld) {
+  if constexpr (sizeof(Real) == sizeof(float)) {
+    // FP32: the flux functions of the explicit kernel (bx_stage_unit.cuh), so
+    // that every FP32 kernel gives the same fluxes; a renaming to the
+    // face's frame at compile time
+    constexpr int T1 = (D + 1) % 3, T2 = (D + 2) % 3;
+    constexpr int var[8] = {0, 1 + D, 1 + T1, 1 + T2, 4 + D, 4 + T1, 4 + T2, 7};
+    auto put = [&](int q, Real f) { out[var[q] * stride] = f; };
+    if constexpr (FLUX == kFluxHlld) {
+      Real l[8], r[8], v;
+#pragma unroll
+      for (int q = 0; q < 8; q++) { l[q] = L[var[q]]; r[q] = R[var[q]]; }
+      const bool ok = hlld_frame(l, r, gamma, invGm1, area, v, put);
+      out[8 * stride] = v;
+      return ok;
+    } else {
+      F2 X[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) X[q] = f2(L[var[q]], R[var[q]]);
+      out[8 * stride] = flux_pair<FLUX>(X, gamma, invGm1, area, put);
+      return true;
+    }
+  } else if constexpr (FLUX == kFluxHlld) {
     Real F[8], v;
     const bool ok = numerical_flux<D, FLUX>(L, R, gamma, invGm1, area, F, v);
 #pragma unroll
     for (int q = 0; q < 8; q++) out[q * stride] = F[q];
     out[8 * stride] = v;
     return ok;
+  } else {
+    out[8 * stride] = flux_lean<D, FLUX>(L, R, gamma, invGm1, area, out, stride);
+    return true;
   }
-  out[8 * stride] = flux_lean<D, FLUX>(L, R, gamma, invGm1, area, out, stride);
-  return true;
 }
 
 // The face states of a face normal to D at index n (0..N) and transverse
@@ -436,7 +466,7 @@ __global__ void __launch_bounds__(T::NTHR, 1)
                           (pb - TileT(0.5) * (prim[m][kUx] * prim[m][kUx] + prim[m][kUy] * prim[m][kUy] +
                                               prim[m][kUz] * prim[m][kUz]) / prim[m][kRho]);
           }
-          const TileT rhoInv = TileT(1) / prim[m][kRho];
+          const TileT rhoInv = cell_rcp(prim[m][kRho]);
           prim[m][kUx] = rhoInv * prim[m][kUx];
           prim[m][kUy] = rhoInv * prim[m][kUy];
           prim[m][kUz] = rhoInv * prim[m][kUz];
@@ -543,7 +573,7 @@ __global__ void __launch_bounds__(T::NTHR, 1)
       if (t == 0) {
         double m = wmin[0];
         for (int w = 1; w < T::NTHR / 32; w++) m = fmin(m, wmin[w]);
-        if (a.dtBlock) a.dtBlock[b] = m;
+        if (a.dtBlock) store_block_dt(a.dtBlock, b, m);
         atomicMin(&a.ts->DtMinBits, (unsigned long long)__double_as_longlong(m));
       }
     }

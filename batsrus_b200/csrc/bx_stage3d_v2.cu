@@ -1,15 +1,20 @@
-// bx_stage3d_v2.cu -- instantiations and launcher of the single-face-phase
-// stage kernel for 8^3 blocks (bx_stage3d_v2.cuh), which the autotuner's
-// stage_variant = 0 selects.
+// bx_stage3d_v2.cu -- instantiations and launchers of the single-face-phase
+// stage kernel for 8^3 blocks (bx_stage3d_v2.cuh): the residual of the
+// implicit step in FP64, and the explicit stages with the Roe flux, whose
+// long face code runs better with one set of barriers per block and 128
+// registers (96^3: 665 us per FP64 step and 368 per FP32-bulk step, against
+// 800 and 420 in units of 128 cells).
+#include "bx_stage3d_launch.cuh"
 #include "bx_stage3d_v2.cuh"
-#include "bx_tune.h"
 
 namespace bx {
 
 namespace {
 
+// one CTA of 512 threads per SM in FP64 (the tile and the face slots fill the
+// shared memory), two of 256 in FP32
 template <int NTHR, int MINB, typename TileT, typename Real, typename OutT, int FLUX, int LIM, bool RC>
-cudaError_t launch8_rc(const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
+cudaError_t launch8(const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
   using B = Blk8<TileT, Real, NTHR, MINB>;
   auto k = stage8_kernel<B, TileT, Real, OutT, FLUX, LIM, RC>;
   constexpr size_t sm = B::smem_bytes;
@@ -19,62 +24,45 @@ cudaError_t launch8_rc(const TmaMaps &maps, const StageArgs &a, int nSM, cudaStr
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  // persistent grid of MINB CTAs per SM (what the shared memory and the
-  // registers of the instantiation hold together)
   const int want = nSM * MINB;
-  const int grid = a.nBlock < want ? a.nBlock : want;
-  k<<<grid, NTHR, sm, st>>>(maps, a);
+  k<<<a.nBlock < want ? a.nBlock : want, NTHR, sm, st>>>(maps, a);
   return cudaGetLastError();
 }
 
-// without the resolution-change face code where no block needs it
-template <int NTHR, int MINB, typename TileT, typename Real, typename OutT, int FLUX, int LIM>
+template <int NTHR, int MINB, typename TileT, typename Real, typename OutT, int FLUX, bool RC>
 cudaError_t launch8_lim(const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
-  if (a.anySpecial) return launch8_rc<NTHR, MINB, TileT, Real, OutT, FLUX, LIM, true>(maps, a, nSM, st);
-  return launch8_rc<NTHR, MINB, TileT, Real, OutT, FLUX, LIM, false>(maps, a, nSM, st);
-}
-
-template <int NTHR, int MINB, typename TileT, typename Real, typename OutT, int FLUX>
-cudaError_t launch8_flux(const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
   switch (a.limiter) {
-    case kLimMinmod: return launch8_lim<NTHR, MINB, TileT, Real, OutT, FLUX, kLimMinmod>(maps, a, nSM, st);
-    case kLimMc: return launch8_lim<NTHR, MINB, TileT, Real, OutT, FLUX, kLimMc>(maps, a, nSM, st);
-    case kLimMc3: return launch8_lim<NTHR, MINB, TileT, Real, OutT, FLUX, kLimMc3>(maps, a, nSM, st);
+    case kLimMinmod: return launch8<NTHR, MINB, TileT, Real, OutT, FLUX, kLimMinmod, RC>(maps, a, nSM, st);
+    case kLimMc: return launch8<NTHR, MINB, TileT, Real, OutT, FLUX, kLimMc, RC>(maps, a, nSM, st);
+    case kLimMc3: return launch8<NTHR, MINB, TileT, Real, OutT, FLUX, kLimMc3, RC>(maps, a, nSM, st);
   }
   return cudaErrorInvalidValue;
 }
 
-template <int NTHR, int MINB, typename TileT, typename Real, typename OutT>
-cudaError_t launch8_kind(int flux, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
-  switch (flux) {
-    case kFluxRusanov: return launch8_flux<NTHR, MINB, TileT, Real, OutT, kFluxRusanov>(maps, a, nSM, st);
-    case kFluxLinde: return launch8_flux<NTHR, MINB, TileT, Real, OutT, kFluxLinde>(maps, a, nSM, st);
-    case kFluxHlld: return launch8_flux<NTHR, MINB, TileT, Real, OutT, kFluxHlld>(maps, a, nSM, st);
-    case kFluxRoe: return launch8_flux<NTHR, MINB, TileT, Real, OutT, kFluxRoe>(maps, a, nSM, st);
+template <bool RC>
+cudaError_t launch8_roe(int kind, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
+  switch (kind) {
+    case kKindFp64: return launch8_lim<512, 1, double, double, double, kFluxRoe, RC>(maps, a, nSM, st);
+    case kKindFp32In64: return launch8_lim<256, 2, double, float, float, kFluxRoe, RC>(maps, a, nSM, st);
+    case kKindFp32In32: return launch8_lim<256, 2, float, float, double, kFluxRoe, RC>(maps, a, nSM, st);
   }
   return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
-cudaError_t launch_stage8(int flux, int kind, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
-  // FP64: one CTA per SM (the FP64 tile and face slots fill the shared
-  // memory) of 512 threads, or 576 (stage_variant 3: three face groups per
-  // warp, 96 registers).  FP32-bulk: one CTA of 512 per SM or, for
-  // stage_ctas_per_sm >= 2, two CTAs of 256, each on its own block
-  const bool two = tune_value(kTuneStageGrid) >= 2;
-  switch (kind) {
-    case kKindFp64:
-      if (tune_value(kTuneStageVariant) == 3) return launch8_kind<576, 1, double, double, double>(flux, maps, a, nSM, st);
-      return launch8_kind<512, 1, double, double, double>(flux, maps, a, nSM, st);
-    case kKindFp32In64:
-      if (two) return launch8_kind<256, 2, double, float, float>(flux, maps, a, nSM, st);
-      return launch8_kind<512, 1, double, float, float>(flux, maps, a, nSM, st);
-    case kKindFp32In32:
-      if (two) return launch8_kind<256, 2, float, float, double>(flux, maps, a, nSM, st);
-      return launch8_kind<512, 1, float, float, double>(flux, maps, a, nSM, st);
+cudaError_t launch_stage8_residual(int flux, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
+  switch (flux) {
+    case kFluxRusanov: return launch8_lim<512, 1, double, double, double, kFluxRusanov, true>(maps, a, nSM, st);
+    case kFluxLinde: return launch8_lim<512, 1, double, double, double, kFluxLinde, true>(maps, a, nSM, st);
+    case kFluxHlld: return launch8_lim<512, 1, double, double, double, kFluxHlld, true>(maps, a, nSM, st);
+    case kFluxRoe: return launch8_lim<512, 1, double, double, double, kFluxRoe, true>(maps, a, nSM, st);
   }
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_stage8_roe(int kind, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
+  return a.anySpecial ? launch8_roe<true>(kind, maps, a, nSM, st) : launch8_roe<false>(kind, maps, a, nSM, st);
 }
 
 }  // namespace bx

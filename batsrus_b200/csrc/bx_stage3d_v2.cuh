@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(B::NTHR, B::MINB)
         w[kP] = (TileT)(a.gamma - 1.0) *
                 (pb - TileT(0.5) * (w[kUx] * w[kUx] + w[kUy] * w[kUy] + w[kUz] * w[kUz]) / w[kRho]);
       }
-      const TileT rhoInv = TileT(1) / w[kRho];
+      const TileT rhoInv = cell_rcp(w[kRho]);
       w[kUx] = rhoInv * w[kUx];
       w[kUy] = rhoInv * w[kUy];
       w[kUz] = rhoInv * w[kUz];
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(B::NTHR, B::MINB)
     if (a.computeDt && t == 0) {
       double m = wmin[0];
       for (int w = 1; w < B::NW; w++) m = fmin(m, wmin[w]);
-      if (a.dtBlock) a.dtBlock[b] = m;
+      if (a.dtBlock) store_block_dt(a.dtBlock, b, m);
       atomicMin(&a.ts->DtMinBits, (unsigned long long)__double_as_longlong(m));
     }
   }

@@ -12,9 +12,9 @@
 
 namespace bx {
 
-static const int g_default[kNumTune] = {2, 4, 2, 1, 192, 0, 3};
+static const int g_default[kNumTune] = {4, 4, 2, 1, 192, 0, 3};
 static TuneKnobInfo g_knobs[kNumTune] = {
-    {"stage_ctas_per_sm", 4, {1, 2, 3, 4}, 2, 0, {}},
+    {"stage_ctas_per_sm", 4, {1, 2, 3, 4}, 4, 0, {}},
     {"krylov_ctas_per_sm", 4, {2, 4, 6, 8}, 4, 0, {}},
     {"krylov_unroll", 3, {1, 2, 4}, 2, 0, {}},
     {"heat_ilu_warps", 3, {1, 2, 4}, 1, 0, {}},

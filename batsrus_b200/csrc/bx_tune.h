@@ -11,12 +11,12 @@
 namespace bx {
 
 enum TuneKnob {
-  kTuneStageGrid = 0,  // persistent stage kernel CTAs per SM (several fit for 4^3 blocks)
+  kTuneStageGrid = 0,  // persistent stage kernel: at most this many CTAs per SM
   kTuneKryCtas,        // Krylov vector kernels: CTAs per SM (256 threads each)
   kTuneKryUnroll,      // Krylov MGS step: independent 16-byte loads in flight per thread and vector
   kTuneHeatIluWarps,   // heat ILU sweeps: warps (groups of 32 blocks) per CTA
   kTuneBiluThreads,    // JFNK BILU sweeps: threads per block CTA (8 per cell of a wavefront)
-  kTuneStageVariant,   // stage kernel, 8^3 blocks: 0 one face phase (FP64: 512 threads, 3: 576); one
+  kTuneStageVariant,   // stage kernel, 8^3 blocks: 0 and 3 units of 128 cells (bx_stage_unit.cuh); one
                        // direction at a time with 1: one face per thread (576 threads), 2: two (288)
   kTuneKryGsSteps,     // Gram-Schmidt steps per pass over w (1 to 4); set, not timed
   kNumTune
