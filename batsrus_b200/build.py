@@ -20,9 +20,8 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
           "--expt-relaxed-constexpr"]
 # (source, extra flags)
 UNITS = [
-    ("bx_stage_fp64.cu", ["--fmad=false"]),
     ("bx_compat.cu", ["--fmad=false"]),
-    ("bx_stage_fp32.cu", []),
+    ("bx_stage_flat.cu", []),
     ("bx_stage3d.cu", []),
     ("bx_stage3d_fpt2.cu", []),
     ("bx_stage3d_v2.cu", []),
@@ -39,7 +38,7 @@ UNITS = [
     ("bx_tune.cu", []),
     ("bx_capi.cu", []),
 ]
-HEADERS = ["bx_physics.cuh", "bx_stage.cuh", "bx_device.h", "bx_stage3d.cuh", "bx_stage3d_v2.cuh", "bx_stage3d_launch.cuh", "bx_stage_unit.cuh",
+HEADERS = ["bx_physics.cuh", "bx_stage.cuh", "bx_device.h", "bx_stage3d.cuh", "bx_stage3d_v2.cuh", "bx_stage3d_launch.cuh", "bx_stage_unit.cuh", "bx_stage_flat.cuh",
            "bx_stage_unit_launch.cuh", "bx_tma.cuh", "bx_core.h",
            "bx_impl_kernels.cuh", "bx_krylov.cuh", "bx_tune.h", "bx_tc.cuh", "bx_learned.cuh", "bx_learned_kernels.cuh", "bx_amr.h"]
 

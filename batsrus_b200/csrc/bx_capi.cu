@@ -68,6 +68,7 @@ struct Ctx {
   cudaStream_t st = nullptr;
   cudaGraphExec_t graph = nullptr;
   double graphTLimit = 0;
+  bool graphFused = false;
   int graphSteps = 1;  // time steps captured in one CUDA graph
   // TMA tensor maps of the two state buffers (3D shapes)
   bool use3d = false;
@@ -179,29 +180,11 @@ __global__ void soa_to_aos(const double *__restrict__ soa, double *__restrict__ 
   }
 }
 
-// set_global_timestep (src/ModTimeStepControl.f90:306-524) on the device
 __global__ void set_dt_kernel(StepState *ts, double tLimit, int useDtFixed, double dtFixed, double cfl) {
-  ts->nStep = ts->nStep + 1;
-  double dt;
-  // BATS_advance always passes a positive limit (tSimulationMax or
-  // huge(0.0)), so the first time-accurate step has Dt = 0
-  if (useDtFixed) dt = dtFixed;
-  else if (ts->nStep <= 1) dt = 0.0;
-  else dt = __longlong_as_double((long long)ts->DtMinBits);
-  if (tLimit > 0.0 && ts->tSimulation + cfl * dt > tLimit) dt = (tLimit - ts->tSimulation) / cfl;
-  ts->DtNoCfl = dt;
-  ts->Dt = cfl * dt;
-  ts->DtMinBits = 0x7FF0000000000000ull;  // +inf
+  step_set_dt(ts, tLimit, useDtFixed, dtFixed, cfl);
 }
 
-// end of BATS_advance: tSimulation += Dt/nStage per stage and the final
-// adjustment to the time limit (src/ModBatsrusMethods.f90:606-640)
-__global__ void end_step_kernel(StepState *ts, int nStage, double tLimit) {
-  double t = ts->tSimulation;
-  for (int s = 0; s < nStage; s++) t = t + ts->Dt / nStage;
-  if (tLimit > 0.0 && t < tLimit && tLimit - t <= 1e-3 * ts->Dt) t = tLimit;
-  ts->tSimulation = t;
-}
+__global__ void end_step_kernel(StepState *ts, int nStage, double tLimit) { step_end(ts, nStage, tLimit); }
 
 __global__ void dtmin_from_blocks(StepState *ts, const double *dtBlock, int nPart) {
   __shared__ double w[32];
@@ -370,9 +353,14 @@ StageArgs stage_args(int iStage, bool computeDt) {
 }
 
 // one stage of all blocks (update_state_fast); the cell time steps are
-// computed in the last stage, or where computeDt asks for them
-int launch_stage_dt(int iStage, bool computeDt) {
+// computed in the last stage, or where computeDt asks for them.  finish:
+// StageArgs::finish, with the time limit tLimit
+int launch_stage_dt(int iStage, bool computeDt, int finish = 0, double tLimit = -1.0) {
   StageArgs a = stage_args(iStage, computeDt);
+  a.finish = finish;
+  a.tLimit = tLimit;
+  a.useDtFixed = g.sch.UseDtFixed;
+  a.dtFixed = g.sch.DtFixed;
   if (g.timing) {
     if (g.nTimed >= (int)g.evStart.size()) {
       cudaEvent_t e0, e1;
@@ -401,10 +389,8 @@ int launch_stage_dt(int iStage, bool computeDt) {
       if (e != cudaSuccess) return fail(BX_ERR_CUDA, "resolution-change kernels: %s", cudaGetErrorString(e));
     }
     e = launch_stage3d(g.shape, g.sch.TypeFlux, kind, *m, a, g.nSM, g.st);
-  } else if (g.sch.Precision == BX_FP64) {
-    e = launch_stage_fp64(g.shape, g.sch.TypeFlux, a, g.st);
   } else {
-    e = launch_stage_fp32(g.shape, g.sch.TypeFlux, iStage == 1 ? 0 : 1, a, g.st);
+    e = launch_stage_flat(g.shape, g.sch.TypeFlux, a, g.st);
   }
   if (e != cudaSuccess) return fail(BX_ERR_CUDA, "stage kernel launch: %s", cudaGetErrorString(e));
   if (g.timing) { CK(cudaEventRecord(g.evStop[g.nTimed], g.st)); g.nTimed++; }
@@ -504,15 +490,34 @@ int tune_stage_impl() {
   return r;
 }
 
-int launch_step(double tLimit) {
+// The time steps of bx_advance.  Where the stage kernel ends the step itself
+// (StageArgs::finish), a step is its stages: begin_steps sets the first
+// one's time step, every step but the last sets the next one's.  Elsewhere
+// each step is launched with its own set_dt and end_step kernels.
+bool fused_steps() { return !g.use3d || stage3d_finishes(g.shape, g.sch.TypeFlux); }
+
+int begin_steps(double tLimit) {
+  if (!fused_steps()) return BX_OK;
   set_dt_kernel<<<1, 1, 0, g.st>>>(g.ts, tLimit, g.sch.UseDtFixed, g.sch.DtFixed, g.sch.Cfl);
   CK(cudaGetLastError());
+  return BX_OK;
+}
+
+int launch_step(double tLimit, bool last) {
+  const bool fused = fused_steps();
+  if (!fused) {
+    set_dt_kernel<<<1, 1, 0, g.st>>>(g.ts, tLimit, g.sch.UseDtFixed, g.sch.DtFixed, g.sch.Cfl);
+    CK(cudaGetLastError());
+  }
   for (int s = 1; s <= g.sch.nStage; s++) {
-    int r = launch_stage(s);
+    const bool end = s == g.sch.nStage;
+    int r = launch_stage_dt(s, end, fused && end ? (last ? 1 : 2) : 0, tLimit);
     if (r) return r;
   }
-  end_step_kernel<<<1, 1, 0, g.st>>>(g.ts, g.sch.nStage, tLimit);
-  CK(cudaGetLastError());
+  if (!fused) {
+    end_step_kernel<<<1, 1, 0, g.st>>>(g.ts, g.sch.nStage, tLimit);
+    CK(cudaGetLastError());
+  }
   return BX_OK;
 }
 
@@ -1195,19 +1200,23 @@ int bx_advance_explicit(int DoCalcTimestep) {
 int bx_advance(int nStep, double tLimit) {
   NEED_READY();
   if (nStep < 0) return fail(BX_ERR_ARG, "nStep=%d", nStep);
+  if (nStep == 0) return check_err_flag();
+  int r = begin_steps(tLimit);
+  if (r) return r;
+  // a graph holds steps that are followed by another one; the last step of
+  // the call is launched directly
   const bool useGraph = !g.timing && g.sch.nStage == 2;
-  if (useGraph && (!g.graph || g.graphTLimit != tLimit) && nStep > 0) {
+  int n = 0;
+  if (useGraph && nStep > 1 && (!g.graph || g.graphTLimit != tLimit || g.graphFused != fused_steps())) {
     // the first step of a new graph runs uncaptured, so that kernel
     // attributes are set before capture begins
-    int r0 = launch_step(tLimit);
-    if (r0) return r0;
-    nStep--;
+    if ((r = launch_step(tLimit, false))) return r;
+    n++;
     if (g.graph) { cudaGraphExecDestroy(g.graph); g.graph = nullptr; }
     cudaGraph_t gr;
     CK(cudaStreamBeginCapture(g.st, cudaStreamCaptureModeThreadLocal));
-    int r = 0;
     for (int q = 0; q < g.graphSteps && !r; q++) {
-      r = launch_step(tLimit);
+      r = launch_step(tLimit, false);
       g.nLaunchTotal -= g.sch.nStage;  // captured, not launched
     }
     cudaError_t e = cudaStreamEndCapture(g.st, &gr);
@@ -1216,15 +1225,15 @@ int bx_advance(int nStep, double tLimit) {
     CK(cudaGraphInstantiate(&g.graph, gr, 0));
     cudaGraphDestroy(gr);
     g.graphTLimit = tLimit;
+    g.graphFused = fused_steps();
   }
-  for (int n = 0; n < nStep;) {
-    if (useGraph && nStep - n >= g.graphSteps) {
+  while (n < nStep) {
+    if (useGraph && g.graph && nStep - 1 - n >= g.graphSteps) {
       CK(cudaGraphLaunch(g.graph, g.st));
       g.nLaunchTotal += g.sch.nStage * g.graphSteps;
       n += g.graphSteps;
     } else {
-      int r = launch_step(tLimit);
-      if (r) return r;
+      if ((r = launch_step(tLimit, n == nStep - 1))) return r;
       n++;
     }
   }

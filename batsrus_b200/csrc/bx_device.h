@@ -22,6 +22,7 @@ struct StepState {
   unsigned long long DtMinBits;   // running min of cell time steps (bits)
   int nStep;
   int errFlag;
+  unsigned nDone;                 // CTAs of the step's last stage that are through (finish_stage)
 };
 
 // Floors of the updated state, each active where > 0: RhoMin_I (the
@@ -48,6 +49,32 @@ __host__ __device__ inline void store_block_dt(double *dt, int b, double m) {
   for (int q = 0; q < kDtParts; q++) dt[(size_t)kDtParts * b + q] = m;
 }
 
+#ifdef __CUDACC__
+// set_global_timestep (src/ModTimeStepControl.f90:306-524) on the device
+__device__ inline void step_set_dt(StepState *ts, double tLimit, int useDtFixed, double dtFixed, double cfl) {
+  ts->nStep = ts->nStep + 1;
+  double dt;
+  // BATS_advance always passes a positive limit (tSimulationMax or
+  // huge(0.0)), so the first time-accurate step has Dt = 0
+  if (useDtFixed) dt = dtFixed;
+  else if (ts->nStep <= 1) dt = 0.0;
+  else dt = __longlong_as_double((long long)ts->DtMinBits);
+  if (tLimit > 0.0 && ts->tSimulation + cfl * dt > tLimit) dt = (tLimit - ts->tSimulation) / cfl;
+  ts->DtNoCfl = dt;
+  ts->Dt = cfl * dt;
+  ts->DtMinBits = 0x7FF0000000000000ull;  // +inf
+}
+
+// end of BATS_advance: tSimulation += Dt/nStage per stage and the final
+// adjustment to the time limit (src/ModBatsrusMethods.f90:606-640)
+__device__ inline void step_end(StepState *ts, int nStage, double tLimit) {
+  double t = ts->tSimulation;
+  for (int s = 0; s < nStage; s++) t = t + ts->Dt / nStage;
+  if (tLimit > 0.0 && t < tLimit && tLimit - t <= 1e-3 * ts->Dt) t = tLimit;
+  ts->tSimulation = t;
+}
+#endif
+
 struct StageArgs {
   const void *in;          // gather source (double* or float*)
   const double *old;       // StateOld: the step's initial state (own cells)
@@ -61,6 +88,11 @@ struct StageArgs {
   int iStage, nStage, nOrder, limiter, useDivb, useHalfStep, computeDt;
   double beta, gamma, invGm1, cfl;
   double dtFactor = 0.0;   // the stage's part of the time step: cfl, or cfl iStage/nStage (half step scheme)
+  // the step's last stage: 0 nothing more, 1 its last CTA ends the time step,
+  // 2 and sets the next one's time step (set_global_timestep)
+  int finish = 0;
+  int useDtFixed = 0;
+  double dtFixed = 0.0, tLimit = -1.0;
   // residual mode of the 3D kernel (get_residual of the implicit scheme):
   // the input holds total energy in the pressure slot, the output is the
   // increment dtScale*DtMax_CB*(S + dF/V) of the implicit variables, with
@@ -91,6 +123,38 @@ struct StageArgs {
   int anySpecial = 1;
 };
 
+#ifdef __CUDACC__
+// The end of a stage kernel, called by every thread of the CTA after its last
+// access to the time-step state: the last CTA through ends the time step and
+// sets the next one's, in place of two launches of one thread each (5 us of
+// a step's 23 on a grid of 16^3).  Every CTA has read DtNoCfl and added its
+// minimum before it counts itself.
+__device__ __forceinline__ void finish_stage(const StageArgs &a) {
+  if (!a.finish) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&a.ts->nDone, 1u) == gridDim.x - 1) {
+      __threadfence();
+      StepState s;
+      s.DtNoCfl = a.ts->DtNoCfl;
+      s.Dt = a.ts->Dt;
+      s.tSimulation = a.ts->tSimulation;
+      s.nStep = a.ts->nStep;
+      s.DtMinBits = atomicAdd(&a.ts->DtMinBits, 0ull);
+      step_end(&s, a.nStage, a.tLimit);
+      if (a.finish == 2) step_set_dt(&s, a.tLimit, a.useDtFixed, a.dtFixed, a.cfl);
+      a.ts->DtNoCfl = s.DtNoCfl;
+      a.ts->Dt = s.Dt;
+      a.ts->tSimulation = s.tSimulation;
+      a.ts->nStep = s.nStep;
+      a.ts->DtMinBits = s.DtMinBits;
+      a.ts->nDone = 0;
+    }
+  }
+}
+#endif
+
 constexpr int kNbrFloat = -1, kNbrResChange = -2;
 constexpr int kRcSlots = 10;
 
@@ -114,11 +178,9 @@ struct CompatArgs {
 // shape ids of the supported block sizes
 enum { kShape888 = 0, kShape444 = 1, kShape881 = 2, kShape811 = 3, kShape6411 = 4, kNumShape = 5 };
 
-// launchers (explicitly instantiated in bx_stage_fp64.cu / bx_stage_fp32.cu
-// / bx_compat.cu)
-cudaError_t launch_stage_fp64(int shape, int flux, const StageArgs &a, cudaStream_t st);
-// kind 0: FP64 in -> FP32 out (stage 1), kind 1: FP32 in -> FP64 out (stage 2)
-cudaError_t launch_stage_fp32(int shape, int flux, int kind, const StageArgs &a, cudaStream_t st);
+// launchers (explicitly instantiated in bx_stage_flat.cu and bx_compat.cu)
+// 1D and 2D blocks
+cudaError_t launch_stage_flat(int shape, int flux, const StageArgs &a, cudaStream_t st);
 cudaError_t launch_compat(int shape, int flux, int phase, int iBlock, const CompatArgs &a,
                           cudaStream_t st);
 // persistent TMA-staged kernel of 3D shapes (bx_stage3d.cu): tensor maps of
@@ -131,6 +193,8 @@ struct alignas(64) TmaMaps {
 enum { kKindFp64 = 0, kKindFp32In64 = 1, kKindFp32In32 = 2 };
 cudaError_t launch_stage3d(int shape, int flux, int kind, const TmaMaps &maps, const StageArgs &a, int nSM,
                            cudaStream_t st);
+// whether that kernel carries out StageArgs::finish
+bool stage3d_finishes(int shape, int flux);
 enum { kPhaseFaceValue = 0, kPhaseFaceFlux = 1, kPhaseSource = 2, kPhaseUpdate = 3, kPhaseTimestep = 4 };
 
 }  // namespace bx

@@ -9,6 +9,11 @@
 
 namespace bx {
 
+bool stage3d_finishes(int shape, int flux) {
+  if (shape == kShape444) return true;
+  return flux != kFluxRoe && (tune_value(kTuneStageVariant) == 0 || tune_value(kTuneStageVariant) == 3);
+}
+
 cudaError_t launch_stage3d(int shape, int flux, int kind, const TmaMaps &maps, const StageArgs &a, int nSM,
                            cudaStream_t st) {
   const int variant = shape == kShape888 ? tune_value(kTuneStageVariant) : 0;

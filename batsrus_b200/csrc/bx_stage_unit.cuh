@@ -565,6 +565,7 @@ __global__ void __launch_bounds__(W::NTHR, W::MINB)
     mbar_wait_bounded(&bar, 0);
     mbar_wait_bounded(&bar, 1);
   }
+  finish_stage(a);
 }
 
 }  // namespace bx
