@@ -52,7 +52,7 @@ bool learned_has_room();
 // the 8 channels (bx_heat.cu)
 int learned_scalar_setup(int nBlock, cudaStream_t st);
 // store block pairs of a scalar solve with the picked blocks' ILU factors
-// (coefL: {lower x, lower y, lower z, 1/pivot} interleaved by 32 blocks):
+// (coefL: {lower x, lower y, lower z, 1/pivot} per cell):
 // the network is then trained on the residual-space loss |M z - t|^2
 int learned_collect_scalar(const double *w, const double *z, const double4 *coefL, const unsigned char *used,
                            int nBlock, cudaStream_t st);

@@ -69,14 +69,10 @@ struct HeatCtx {
   double *K = nullptr;  // face conduction tensor [block][dim][dir][face]
   float *K32 = nullptr; // the same in FP32 for the matrix-free product (op32)
   bool op32 = false;    // OperatorPrecision = BX_FP32_BULK
-  void *coef = nullptr;      // forward and backward sweep coefficients (double4 or float4), interleaved by 32 blocks
-  void *yI = nullptr;        // forward-sweep scratch (double or float), interleaved
-  bool ilu32 = false;        // FP32 coefficients, scratch and sweep arithmetic
+  void *coef = nullptr;      // sweep coefficients [block][cell] (double4 or float4)
+  bool ilu32 = false;        // FP32 coefficients and sweep arithmetic
   double *V8 = nullptr, *Z8 = nullptr;  // learned preconditioner: embedded input and output [block][8][512]
   double *Zb = nullptr;                 // flexible GMRES: preconditioned basis (m vectors)
-  unsigned *usedM = nullptr; // used masks [group][cell]
-  int nGroup = 0;            // groups of 32 blocks
-  long nIl = 0;              // cells of the interleaved arrays (nGroup x 32 x 512)
   struct WaveTable *wtab = nullptr;
   unsigned *cnt = nullptr;
   int *errDev = nullptr;  // device error flag of the bounded waits
@@ -293,18 +289,14 @@ __global__ void __launch_bounds__(512) k_heat_apply(HeatArgs a, const double *__
 // holds the couplings to the -x, -y, -z neighbours and the diagonal, which
 // the factorisation replaces by the ILU(0) pivot.  Couplings across block
 // faces and to unused cells are dropped (BILU on 8^3 blocks).  The sweeps
-// multiply by the pivot reciprocals that the factorisation stores.  Per
-// cell the factorisation writes two double4: {lower x, lower y, lower z,
-// 1/pivot} for the forward sweep and {upper x, upper y, upper z, 1/pivot}
-// (the lower couplings of the +x, +y, +z neighbours) for the backward one.
+// multiply by the pivot reciprocals that the factorisation stores: one
+// double4 or float4 per cell, {lower x, lower y, lower z, 1/pivot}, with zero
+// couplings across block faces and next to unused cells, so that the sweeps
+// need no masks.  The backward sweep reads the same four numbers: the upper
+// couplings of a cell are the lower ones of its +x, +y, +z neighbours.
 //
-// The factorisation runs one warp per block over the 22 planes i+j+k =
-// const (every lower neighbour lies on the previous plane).  The sweeps run
-// one lane per block in the natural order of the oracle, 32 blocks per warp
-// with no barrier between cells: the coefficients and the used flags are
-// stored interleaved by groups of 32 blocks (a warp's load of one cell of its
-// 32 blocks is one contiguous 1 KB), and the right-hand side and the result
-// pass through a shared-memory transpose one 8x8 plane at a time.
+// The factorisation and the sweeps run one warp per block over the 22 planes
+// i+j+k = const (every lower neighbour lies on the previous plane).
 constexpr int kWarpsPerCta = 2, kNumWave = 3 * (kNB - 1) + 1;
 
 struct WaveTable {
@@ -330,13 +322,13 @@ __device__ __forceinline__ void put4(float4 *p, double x, double y, double z, do
   *p = make_float4((float)x, (float)y, (float)z, (float)w);
 }
 
-// matrix + factorisation (FP64); coef[q] = {lower x, lower y, lower z,
-// 1 / pivot}, stored as double4 or, for the FP32 sweeps, float4
+// matrix + factorisation (FP64); coef[block][cell] = {lower x, lower y,
+// lower z, 1 / pivot}, stored as double4 or, for the FP32 sweeps, float4
 template <typename C4>
 __global__ void __launch_bounds__(32 * kWarpsPerCta) k_heat_factor(HeatArgs a, const double *__restrict__ K,
                                                                  const unsigned char *__restrict__ used,
-                                                                 const WaveTable *__restrict__ wtab, C4 *coefL,
-                                                                 C4 *coefU, int nBlock) {
+                                                                 const WaveTable *__restrict__ wtab, C4 *coef,
+                                                                 int nBlock) {
   __shared__ IluSmem sm;
   load_wave_table(wtab, sm.wt);
   __syncthreads();
@@ -386,158 +378,137 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) k_heat_factor(HeatArgs a, c
     __syncwarp();
   }
   for (int c = lane; c < kNC; c += 32) {
-    const double iv = 1.0 / dp[c];
-    const long o = ((long)(blk >> 5) * kNC + c) * 32 + (blk & 31);  // interleaved by 32 blocks
-    put4(coefL + o, lx[c], ly[c], lz[c], iv);
-    put4(coefU + o, (c & 7) != 7 ? lx[c + 1] : 0.0, ((c >> 3) & 7) != 7 ? ly[c + 8] : 0.0,
-         (c >> 6) != 7 ? lz[c + 64] : 0.0, iv);
+    const bool uc = u[c];
+    put4(coef + (long)blk * kNC + c, (uc && (c & 7) && u[c - 1]) ? lx[c] : 0.0,
+         (uc && ((c >> 3) & 7) && u[c - 8]) ? ly[c] : 0.0, (uc && (c >> 6) && u[c - 64]) ? lz[c] : 0.0, 1.0 / dp[c]);
   }
 }
 
-// z = M^-1 r: forward sweep (L + D) y = r, backward (D + U) z = D y, one
-// lane per block (blocks 32 g .. 32 g + 31 in warp g); usedM[g][c] has bit
-// l set when cell c of block 32 g + l is used; yI is the interleaved
-// scratch of the forward result.  Plane buffers hold element (p, l) at
-// p * 32 + (l ^ (p & 31)): rows and columns are free of bank conflicts.
-__device__ __forceinline__ int swz(int p, int l) { return p * 32 + (l ^ (p & 31)); }
-
+// z = M^-1 r: forward sweep (L + D) y = r, backward (D + U) z = D y, one warp
+// per block.  Lane l owns the two columns of 8 cells along x at (j, k) =
+// (l % 8, l / 8) and (l % 8, l / 8 + 4): cells 8 l + i and 8 l + 256 + i.  Step w
+// of a sweep takes cell i = w - j - k of each column where there is one: its
+// x neighbour is the lane's own previous cell, its y and z neighbours are
+// the cells that lanes l - 1 and l - 8 (forward; l + 1 and l + 8 backward)
+// took one step earlier, so they come by shuffles, and no barrier separates
+// the steps.  The block's coefficients and vector lie in shared memory in
+// their natural order: at a step the lanes of a quarter warp have distinct
+// i, so the 16-byte loads of the coefficients are free of bank conflicts.
+//
+// Bytes per cell: coefficients 16 (FP32; FP64 32), r and z 16.  What bounds
+// it is the latency of the 44 steps on small grids and these bytes on large
+// ones; a lane per block (32 blocks per warp in natural order, interleaved
+// coefficients for both sweeps and a scratch vector, 56 bytes per cell) left
+// all but one warp per SM idle at 128^3 and took 229 us there; now 19 us.
+// W warps per CTA (autotuned); T is the type of the coefficients and the
+// arithmetic (r and z are FP64).
 template <typename T> struct Vec4T;
 template <> struct Vec4T<double> { using type = double4; };
 template <> struct Vec4T<float> { using type = float4; };
 
-template <typename T>
-struct IluRow {
-  typename Vec4T<T>::type v[kNB];
-  unsigned m[kNB];
-};
-
-__device__ __forceinline__ double4 ldg4(const double4 *p) {
-  const double2 *p2 = reinterpret_cast<const double2 *>(p);
-  const double2 lo = __ldg(p2), hi = __ldg(p2 + 1);
-  return make_double4(lo.x, lo.y, hi.x, hi.y);
-}
-__device__ __forceinline__ float4 ldg4(const float4 *p) { return __ldg(p); }
-
-// the coefficients and used masks of one x row (8 cells from c0), loaded
-// ahead of the row's arithmetic
-template <typename T>
-__device__ __forceinline__ void load_row(IluRow<T> &row, const typename Vec4T<T>::type *__restrict__ cf,
-                                         const unsigned *__restrict__ um, int c0) {
-#pragma unroll
-  for (int i = 0; i < kNB; i++) {
-    row.v[i] = ldg4(cf + (long)(c0 + i) * 32);
-    row.m[i] = __ldg(um + c0 + i);
-  }
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-// W warps per CTA (autotuned), each with its own group of 32 blocks and
-// its two plane buffers (32 KB in FP64, 16 KB in FP32) in dynamic shared
-// memory; T is the type of the coefficients, the scratch and the
-// arithmetic (r and z are FP64)
 template <int W, typename T>
-__global__ void __launch_bounds__(32 * W) k_heat_ilu(const typename Vec4T<T>::type *__restrict__ coefL,
-                                                     const typename Vec4T<T>::type *__restrict__ coefU,
-                                                     const unsigned *__restrict__ usedM,
-                                                     const double *__restrict__ r, T *__restrict__ yI,
-                                                     double *__restrict__ z, int nBlock, int nGroup) {
+__global__ void __launch_bounds__(32 * W) k_heat_ilu(const typename Vec4T<T>::type *__restrict__ coef,
+                                                     const double *__restrict__ r, double *__restrict__ z,
+                                                     int nBlock) {
   using V4 = typename Vec4T<T>::type;
   extern __shared__ __align__(16) unsigned char dynb[];
   const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = blockIdx.x * W + wp;
-  if (g >= nGroup) return;  // the warps work independently (no CTA barrier)
-  T(*plane)[64 * 32] = reinterpret_cast<T(*)[64 * 32]>(dynb + sizeof(T) * (size_t)wp * 2 * 64 * 32);
-  const long gb = (long)g * 32;  // first block of the group
-  const unsigned *um = usedM + (long)g * kNC;
-  const V4 *cL = coefL + (long)g * kNC * 32 + lane, *cU = coefU + (long)g * kNC * 32 + lane;
-  T *yl = yI + (long)g * kNC * 32 + lane;
-  T *cur = plane[0], *prv = plane[1];
-  IluRow<T> A, B;
-  // forward, rows (j, k) in natural order
-  load_row(A, cL, um, 0);
-  for (int k = 0; k < kNB; k++) {
-#pragma unroll 8
-    for (int bb = 0; bb < 32; bb++) {
-      const long blk = gb + bb;
-      T v0 = T(0), v1 = T(0);
-      if (blk < nBlock) {
-        v0 = (T)__ldg(r + blk * kNC + 64 * k + lane);
-        v1 = (T)__ldg(r + blk * kNC + 64 * k + 32 + lane);
-      }
-      cur[swz(lane, bb)] = v0;
-      cur[swz(32 + lane, bb)] = v1;
-    }
-    __syncwarp();
-    unsigned mDn[kNB] = {0, 0, 0, 0, 0, 0, 0, 0};  // masks of the row below
-    for (int j = 0; j < kNB; j++) {
-      const int c0 = 64 * k + 8 * j;
-      if (c0 + 8 < kNC) load_row(B, cL, um, c0 + 8);
-      T ym = T(0);  // y of the cell at x - 1
+  const long blk = (long)blockIdx.x * W + wp;
+  if (blk >= nBlock) return;  // the warps work independently (no CTA barrier)
+  V4 *cf = reinterpret_cast<V4 *>(dynb + (sizeof(V4) + sizeof(T)) * kNC * wp);
+  T *y = reinterpret_cast<T *>(cf + kNC);
+  {
+    constexpr int kChunks = sizeof(V4) * kNC / 16 / 32;
+    const char *src = reinterpret_cast<const char *>(coef + blk * kNC);
+    char *dst = reinterpret_cast<char *>(cf);
 #pragma unroll
-      for (int i = 0; i < kNB; i++) {
-        const int p = i + 8 * j, c = c0 + i;
-        const unsigned m = A.m[i];
-        const V4 v = A.v[i];
-        T s = cur[swz(p, lane)];
-        if ((m >> lane) & 1) {
-          if (i > 0 && ((A.m[i - 1] >> lane) & 1)) s = s - v.x * ym;
-          if (j > 0 && ((mDn[i] >> lane) & 1)) s = s - v.y * cur[swz(p - 8, lane)];
-          if (k > 0 && ((__ldg(um + c - 64) >> lane) & 1)) s = s - v.z * prv[swz(p, lane)];
-        }
-        const T y = s * v.w;
-        cur[swz(p, lane)] = y;
-        yl[(long)c * 32] = y;
-        ym = y;
-      }
+    for (int q = 0; q < kChunks; q++) cp_async16(dst + 16 * (32 * q + lane), src + 16 * (32 * q + lane));
+    const double2 *r2 = reinterpret_cast<const double2 *>(r + blk * kNC);
+    double2 v[kNC / 64];
 #pragma unroll
-      for (int i = 0; i < kNB; i++) mDn[i] = A.m[i];
-      A = B;
+    for (int q = 0; q < kNC / 64; q++) v[q] = __ldg(r2 + 32 * q + lane);
+#pragma unroll
+    for (int q = 0; q < kNC / 64; q++) {
+      y[64 * q + 2 * lane] = (T)v[q].x;
+      y[64 * q + 2 * lane + 1] = (T)v[q].y;
     }
-    __syncwarp();
-    T *t = cur; cur = prv; prv = t;
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   __syncwarp();
-  // backward, rows in reverse order
-  load_row(A, cU, um, kNC - 8);
-  for (int k = kNB - 1; k >= 0; k--) {
-    unsigned mUp[kNB] = {0, 0, 0, 0, 0, 0, 0, 0};  // masks of the row above
-    for (int j = kNB - 1; j >= 0; j--) {
-      const int c0 = 64 * k + 8 * j;
-      if (c0 > 0) load_row(B, cU, um, c0 - 8);
-      T yv[kNB];
-#pragma unroll
-      for (int i = 0; i < kNB; i++) yv[i] = yl[(long)(c0 + i) * 32];
-      T zp = T(0);  // z of the cell at x + 1
-#pragma unroll
-      for (int i = kNB - 1; i >= 0; i--) {
-        const int p = i + 8 * j, c = c0 + i;
-        const unsigned m = A.m[i];
-        const V4 v = A.v[i];
-        T s = T(0);
-        if ((m >> lane) & 1) {
-          if (i < kNB - 1 && ((A.m[i + 1] >> lane) & 1)) s = s + v.x * zp;
-          if (j < kNB - 1 && ((mUp[i] >> lane) & 1)) s = s + v.y * cur[swz(p + 8, lane)];
-          if (k < kNB - 1 && ((__ldg(um + c + 64) >> lane) & 1)) s = s + v.z * prv[swz(p, lane)];
-        }
-        const T zc = yv[i] - s * v.w;
-        cur[swz(p, lane)] = zc;
-        zp = zc;
-      }
-#pragma unroll
-      for (int i = 0; i < kNB; i++) mUp[i] = A.m[i];
-      A = B;
+  const int j = lane & 7, ka = lane >> 3, c0 = 8 * lane;
+  // forward: y = (r - lx y(x-1) - ly y(y-1) - lz y(z-1)) / pivot; a column's
+  // value is 0 before its first cell, where the couplings are zero anyway
+  T ya = T(0), yb = T(0);
+#pragma unroll 2
+  for (int w = 0; w < kNumWave; w++) {
+    const int ia = w - j - ka, ib = ia - 4;
+    const T pya = __shfl_sync(0xffffffffu, ya, (lane - 1) & 31), pyb = __shfl_sync(0xffffffffu, yb, (lane - 1) & 31);
+    // z - 1 of the first column's plane k = 0 has no coupling; that of the
+    // second column's first plane is the first column's last one
+    const T pza = __shfl_sync(0xffffffffu, ya, (lane - 8) & 31);
+    const T pzb = __shfl_sync(0xffffffffu, lane >= 24 ? ya : yb, (lane - 8) & 31);
+    if ((unsigned)ia < 8u) {
+      const V4 v = cf[c0 + ia];
+      T s = y[c0 + ia];
+      s = s - v.x * ya;
+      s = s - v.y * pya;
+      s = s - v.z * pza;
+      ya = s * v.w;
+      y[c0 + ia] = ya;
     }
-    __syncwarp();
-#pragma unroll 8
-    for (int bb = 0; bb < 32; bb++) {
-      const long blk = gb + bb;
-      if (blk < nBlock) {
-        z[blk * kNC + 64 * k + lane] = (double)cur[swz(lane, bb)];
-        z[blk * kNC + 64 * k + 32 + lane] = (double)cur[swz(32 + lane, bb)];
-      }
+    if ((unsigned)ib < 8u) {
+      const V4 v = cf[c0 + 256 + ib];
+      T s = y[c0 + 256 + ib];
+      s = s - v.x * yb;
+      s = s - v.y * pyb;
+      s = s - v.z * pzb;
+      yb = s * v.w;
+      y[c0 + 256 + ib] = yb;
     }
-    __syncwarp();
-    T *t = cur; cur = prv; prv = t;
   }
+  // backward: z = y - (ux z(x+1) + uy z(y+1) + uz z(z+1)) / pivot; a cell
+  // hands its neighbours below the products with its own lower couplings
+  T xa = T(0), xb = T(0), qa = T(0), qb = T(0), ta = T(0), tb = T(0);  // products for x - 1, y - 1, z - 1
+#pragma unroll 2
+  for (int w = kNumWave - 1; w >= 0; w--) {
+    const int ia = w - j - ka, ib = ia - 4;
+    const T pya = __shfl_sync(0xffffffffu, qa, (lane + 1) & 31), pyb = __shfl_sync(0xffffffffu, qb, (lane + 1) & 31);
+    // z + 1 of the first column's last plane is the second column's first one;
+    // the second column's last plane is the block's
+    const T pzb = __shfl_sync(0xffffffffu, tb, (lane + 8) & 31);
+    const T pza = __shfl_sync(0xffffffffu, lane < 8 ? tb : ta, (lane + 8) & 31);
+    if ((unsigned)ia < 8u) {
+      const V4 v = cf[c0 + ia];
+      T s = xa;
+      if (j < 7) s = s + pya;
+      s = s + pza;
+      const T zc = y[c0 + ia] - s * v.w;
+      y[c0 + ia] = zc;
+      xa = v.x * zc;
+      qa = v.y * zc;
+      ta = v.z * zc;
+    }
+    if ((unsigned)ib < 8u) {
+      const V4 v = cf[c0 + 256 + ib];
+      T s = xb;
+      if (j < 7) s = s + pyb;
+      if (ka < 3) s = s + pzb;
+      const T zc = y[c0 + 256 + ib] - s * v.w;
+      y[c0 + 256 + ib] = zc;
+      xb = v.x * zc;
+      qb = v.y * zc;
+      tb = v.z * zc;
+    }
+  }
+  __syncwarp();
+  double2 *z2 = reinterpret_cast<double2 *>(z + blk * kNC);
+#pragma unroll
+  for (int q = 0; q < kNC / 64; q++)
+    z2[32 * q + lane] = make_double2((double)y[64 * q + 2 * lane], (double)y[64 * q + 2 * lane + 1]);
 }
 
 WaveTable make_wave_table() {
@@ -563,7 +534,7 @@ __global__ void k_h_te_update(double *Te, const double *x, const unsigned char *
 template <int W, typename T>
 cudaError_t launch_ilu_wt(const double *r, double *z, cudaStream_t st) {
   using V4 = typename Vec4T<T>::type;
-  constexpr size_t smem = sizeof(T) * W * 2 * 64 * 32;
+  constexpr size_t smem = (sizeof(V4) + sizeof(T)) * kNC * W;
   static bool attr = false;
   if (!attr) {
     const cudaError_t e =
@@ -571,9 +542,7 @@ cudaError_t launch_ilu_wt(const double *r, double *z, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  const V4 *cf = static_cast<const V4 *>(H.coef);
-  k_heat_ilu<W, T><<<(H.nGroup + W - 1) / W, 32 * W, smem, st>>>(cf, cf + H.nIl, H.usedM, r, static_cast<T *>(H.yI),
-                                                                  z, H.nBlock, H.nGroup);
+  k_heat_ilu<W, T><<<(H.nBlock + W - 1) / W, 32 * W, smem, st>>>(static_cast<const V4 *>(H.coef), r, z, H.nBlock);
   return cudaGetLastError();
 }
 
@@ -586,13 +555,10 @@ cudaError_t launch_ilu_w(const double *r, double *z, cudaStream_t st) {
 // sweeps' precision)
 void launch_factor(cudaStream_t st) {
   const int grid = (H.nBlock + kWarpsPerCta - 1) / kWarpsPerCta;
-  if (H.ilu32) {
-    float4 *cf = static_cast<float4 *>(H.coef);
-    k_heat_factor<<<grid, 32 * kWarpsPerCta, 0, st>>>(H.a, H.K, H.used, H.wtab, cf, cf + H.nIl, H.nBlock);
-  } else {
-    double4 *cf = static_cast<double4 *>(H.coef);
-    k_heat_factor<<<grid, 32 * kWarpsPerCta, 0, st>>>(H.a, H.K, H.used, H.wtab, cf, cf + H.nIl, H.nBlock);
-  }
+  if (H.ilu32)
+    k_heat_factor<<<grid, 32 * kWarpsPerCta, 0, st>>>(H.a, H.K, H.used, H.wtab, static_cast<float4 *>(H.coef), H.nBlock);
+  else
+    k_heat_factor<<<grid, 32 * kWarpsPerCta, 0, st>>>(H.a, H.K, H.used, H.wtab, static_cast<double4 *>(H.coef), H.nBlock);
 }
 
 cudaError_t launch_ilu(int w, const double *r, double *z, cudaStream_t st) {
@@ -660,10 +626,6 @@ void free_heat() {
     if (*p) cudaFree(*p);
     *p = nullptr;
   }
-  if (H.yI) cudaFree(H.yI);
-  if (H.usedM) cudaFree(H.usedM);
-  H.yI = nullptr;
-  H.usedM = nullptr;
   if (H.coef) cudaFree(H.coef);
   if (H.wtab) cudaFree(H.wtab);
   if (H.cnt) cudaFree(H.cnt);
@@ -1072,12 +1034,9 @@ int bx_heat_init(const bx_heat_params *prm, const double *Te, const double *bhat
   const size_t vb = sizeof(double) * H.nCell;
   bool ok = true;
   for (double **p : {&H.Te, &H.HC, &H.b, &H.x, &H.w, &H.t, &H.r}) ok = ok && cudaMalloc(p, vb) == cudaSuccess;
-  H.nGroup = (H.nBlock + 31) / 32;
-  H.nIl = (long)H.nGroup * 32 * kNC;
+  const size_t cfBytes = (H.ilu32 ? sizeof(float4) : sizeof(double4)) * H.nCell;
   ok = ok && cudaMalloc(&H.B3, 3 * vb) == cudaSuccess &&
-       cudaMalloc(&H.coef, 2 * (H.ilu32 ? sizeof(float4) : sizeof(double4)) * H.nIl) == cudaSuccess &&
-       cudaMalloc(&H.yI, (H.ilu32 ? sizeof(float) : sizeof(double)) * H.nIl) == cudaSuccess &&
-       cudaMalloc(&H.usedM, sizeof(unsigned) * H.nGroup * kNC) == cudaSuccess &&
+       cudaMalloc(&H.coef, cfBytes) == cudaSuccess &&
        cudaMalloc(&H.K, sizeof(double) * kKBlock * H.nBlock) == cudaSuccess &&
        (!H.op32 || cudaMalloc(&H.K32, sizeof(float) * kKBlock * H.nBlock) == cudaSuccess) &&
        cudaMalloc(&H.wtab, sizeof(WaveTable)) == cudaSuccess && cudaMalloc(&H.cnt, sizeof(unsigned)) == cudaSuccess &&
@@ -1110,14 +1069,6 @@ int bx_heat_init(const bx_heat_params *prm, const double *Te, const double *bhat
                            (int)apply_smem<double>()));
   CKH(cudaFuncSetAttribute(k_heat_apply<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)apply_smem<float>()));
-  CKH(cudaMemsetAsync(H.coef, 0, 2 * (H.ilu32 ? sizeof(float4) : sizeof(double4)) * H.nIl, c.st));
-  {
-    std::vector<unsigned> um((size_t)H.nGroup * kNC, 0u);
-    for (long b = 0; b < H.nBlock; b++)
-      for (int q = 0; q < kNC; q++)
-        if (used[b * kNC + q]) um[(size_t)(b >> 5) * kNC + q] |= 1u << (b & 31);
-    CKH(cudaMemcpy(H.usedM, um.data(), sizeof(unsigned) * um.size(), cudaMemcpyHostToDevice));
-  }
   if (const int e = update_coef(c.st)) return e;
   CKH(cudaGetLastError());
   CKH(cudaStreamSynchronize(c.st));

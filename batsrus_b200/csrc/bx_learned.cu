@@ -201,13 +201,12 @@ __global__ void k_collect(const double *__restrict__ w, const double *__restrict
 }
 
 // the ILU factors of the picked blocks of a scalar solve: coefL is the
-// forward-sweep double4 {lower x, lower y, lower z, 1/pivot} per cell,
-// interleaved by groups of 32 blocks; the couplings are kept where the cell
-// and its neighbour are both used
+// sweep double4 {lower x, lower y, lower z, 1/pivot} per cell; the couplings
+// are kept where the cell and its neighbour are both used
 __global__ void k_collect_mc(const double4 *__restrict__ coefL, const unsigned char *__restrict__ used,
                              const int *__restrict__ pick, long base, float4 *mcoef) {
   const int b = pick[blockIdx.x], c = threadIdx.x;
-  const double4 v = coefL[((size_t)(b >> 5) * 512 + c) * 32 + (b & 31)];
+  const double4 v = coefL[(size_t)b * 512 + c];
   const unsigned char *u = used + (size_t)b * 512;
   const int i = c & 7, j = (c >> 3) & 7, k = c >> 6;
   const bool uc = u[c];
