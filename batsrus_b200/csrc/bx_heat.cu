@@ -76,7 +76,7 @@ struct HeatCtx {
   struct WaveTable *wtab = nullptr;
   unsigned *cnt = nullptr;
   int *errDev = nullptr;  // device error flag of the bounded waits
-  double *partial = nullptr, *scal = nullptr;
+  double *partial = nullptr, *scal = nullptr, *gram = nullptr;
   int nMatvec = 0;
   double errRel = 0;
   cudaEvent_t ev[2] = {};
@@ -608,7 +608,7 @@ __global__ void k_heat_take0(const double *__restrict__ Z8, double *z, long n) {
 }
 
 void free_heat() {
-  for (double **p : {&H.Te, &H.HC, &H.B3, &H.b, &H.x, &H.w, &H.t, &H.r, &H.V, &H.partial, &H.scal}) {
+  for (double **p : {&H.Te, &H.HC, &H.B3, &H.b, &H.x, &H.w, &H.t, &H.r, &H.V, &H.partial, &H.scal, &H.gram}) {
     if (*p) cudaFree(*p);
     *p = nullptr;
   }
@@ -739,7 +739,7 @@ int gmres(int &iError, cudaStream_t st) {
       if ((r = matvec(Vk, H.t, st))) return r;
       if ((r = precond(H.t, H.w, st))) return r;
       if (H.p.TypePrecond == BX_PRECOND_BILU && learned_collecting() && (r = collect_pair(H.t, H.w, st))) return r;
-      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.partial, H.cnt, st);  // scal 160..177
+      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, st);  // scal 160..177
       CKH(cudaGetLastError());
       CKH(cudaMemcpyAsync(hb.data(), hdev, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, st));
       CKH(cudaStreamSynchronize(st));
@@ -824,7 +824,7 @@ int fgmres(int &iError, cudaStream_t st) {
       double *Vk = Vb + (size_t)k * N, *Zk = Zb + (size_t)k * N;
       if ((r = precond(Vk, Zk, st))) return r;
       if ((r = matvec(Zk, H.w, st))) return r;
-      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.partial, H.cnt, st);  // scal 160..177
+      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, st);  // scal 160..177
       CKH(cudaGetLastError());
       CKH(cudaMemcpyAsync(hb.data(), hdev, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, st));
       CKH(cudaStreamSynchronize(st));
@@ -1045,7 +1045,8 @@ int bx_heat_init(const bx_heat_params *prm, const double *Te, const double *bhat
        cudaMalloc(&H.used, H.nCell) == cudaSuccess &&
        cudaMalloc(&H.blkAt, sizeof(int) * atH.size()) == cudaSuccess &&
        cudaMalloc(&H.blkXYZ, sizeof(int) * xyzH.size()) == cudaSuccess &&
-       cudaMalloc(&H.partial, sizeof(double) * 10 * kKryMaxBlocks) == cudaSuccess &&
+       cudaMalloc(&H.partial, sizeof(double) * kKryPartials * kKryMaxBlocks) == cudaSuccess &&
+       cudaMalloc(&H.gram, sizeof(double) * kKryGramLd * kKryGramLd) == cudaSuccess &&
        cudaMalloc(&H.scal, sizeof(double) * 192) == cudaSuccess;
   if (!ok) {
     free_heat();

@@ -44,6 +44,7 @@ struct ImplCtx {
   double *jacPre = nullptr;                    // k_jac_cells terms when the Krylov basis V is too small
   int precKind = BX_FP64;                      // factor storage: BX_FP64, BX_FP32_BULK, BX_BF16_FACTORS
   double *partial = nullptr, *scal = nullptr;  // reduction scratch, device scalars
+  double *gram = nullptr;                      // Gram matrix of the Krylov basis
   unsigned *cnt = nullptr;                     // CTA counter of the one-launch reductions
   double *dNorm = nullptr;
   int *wfCell = nullptr, *wfStart = nullptr, *wfPos = nullptr;
@@ -85,7 +86,7 @@ void by_storage(int nI, Fn fn) {
 
 void free_impl() {
   for (double **p : {&I.U, &I.Uold, &I.ResExpl, &I.ResImpl, &I.Rhs, &I.X, &I.Ueps, &I.Reps, &I.W, &I.R, &I.V,
-                     &I.Z, &I.dtCell, &I.partial, &I.scal, &I.dNorm, &I.jacPre}) {
+                     &I.Z, &I.dtCell, &I.partial, &I.scal, &I.dNorm, &I.jacPre, &I.gram}) {
     if (*p) cudaFree(*p);
     *p = nullptr;
   }
@@ -225,7 +226,7 @@ int gmres(int &iError) {
       if ((r = precond(Vk, Zk))) return r;
       if (learned_collecting() && c.nI == 8 && (r = learned_collect(Vk, Zk, c.nBlock, c.st))) return r;
       if ((r = matvec(Zk, I.W))) return r;
-      kry_orth(I.W, I.V, k, N, hdev, I.scal + 104, I.partial, I.cnt, c.st);  // scal 104..121
+      kry_orth(I.W, I.V, k, N, hdev, I.scal + 104, I.gram, I.partial, I.cnt, c.st);  // scal 104..121
       CKI(cudaGetLastError());
       CKI(cudaMemcpyAsync(hb.data(), hdev, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, c.st));
       CKI(cudaStreamSynchronize(c.st));
@@ -386,7 +387,8 @@ int bx_implicit_init(const bx_implicit_params *prm) {
     if (cudaMalloc(p, vb) != cudaSuccess) { free_impl(); return core_fail(BX_ERR_NOMEM, "implicit vectors"); }
   if (cudaMalloc(&I.V, vb * (I.m + 1)) != cudaSuccess || cudaMalloc(&I.Z, vb * I.m) != cudaSuccess ||
       cudaMalloc(&I.dtCell, sizeof(double) * I.nCellTot) != cudaSuccess ||
-      cudaMalloc(&I.partial, sizeof(double) * (kRedBlocks * 8 > 10 * kKryMaxBlocks ? kRedBlocks * 8 : 10 * kKryMaxBlocks)) != cudaSuccess ||
+      cudaMalloc(&I.partial, sizeof(double) * std::max(kRedBlocks * 8, kKryPartials * kKryMaxBlocks)) != cudaSuccess ||
+      cudaMalloc(&I.gram, sizeof(double) * kKryGramLd * kKryGramLd) != cudaSuccess ||
       cudaMalloc(&I.scal, sizeof(double) * 128) != cudaSuccess || cudaMalloc(&I.dNorm, sizeof(double) * 8) != cudaSuccess ||
       cudaMalloc(&I.cnt, sizeof(unsigned)) != cudaSuccess || cudaMemset(I.cnt, 0, sizeof(unsigned)) != cudaSuccess) {
     free_impl();

@@ -319,15 +319,197 @@ inline void kry_gs(const GsArgs &a, int na, int nc, cudaStream_t st) {
   }
 }
 
+// All Gram-Schmidt steps of an Arnoldi column in two passes.
+//   k_kry_dots: the inner products d_i = w . V_i (i = 0..k) and the newest
+//     column of the Gram matrix, G_ik = V_i . V_k (i < k), in one pass over the
+//     basis; its last CTA finishes the sums in a fixed order and takes the
+//     coefficients of modified Gram-Schmidt by forward substitution,
+//     c_j = d_j - sum_{i<j} c_i G_ij (the inverse compact WY form of
+//     low-synchronisation GMRES, Swirydowicz, Langou, Ananthan, Yang and
+//     Thomas 2020), into h[0..k];
+//   k_kry_sub: w -= sum c_i V_i in the order of i, and h[k+1] = w . w.
+// Per column 2 (k + 1) + 4 vectors cross HBM where S steps per pass take
+// 2 (k + 1) + 2 (k + 1) / S + 1 and as many launches.  A thread keeps four
+// 16-byte pieces of w and V_k in registers while it runs over the basis, the
+// next vector's loads in flight behind the current sums; each warp's two sums
+// of a vector are folded into one butterfly (lane 0 ends with d, lane 1 with G).
+constexpr int kKryAllSteps = 64;  // value of kTuneKryGsSteps
+constexpr int kKryGramLd = 65;                                  // basis of at most 65 vectors
+constexpr int kKryPieces = 4, kKryTile = kKryThreads * kKryPieces;  // double2 per tile
+constexpr int kKryPartials = 2 * kKryGramLd;                    // sums per CTA
+
+inline int kry_pass_grid(long n) {
+  const long tiles = (n / 2 + kKryTile - 1) / kKryTile;
+  int dev = 0, nsm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const long want = 2l * nsm < kKryMaxBlocks ? 2l * nsm : kKryMaxBlocks;
+  return (int)(tiles < want ? tiles : want);
+}
+
+static __global__ void __launch_bounds__(kKryThreads, 2)
+    k_kry_dots(const double *__restrict__ w, const double *__restrict__ V, int k, long n, double *partial, unsigned *cnt,
+               double *gram, double *h) {
+  __shared__ double acc[kKryPartials][kKryThreads / 32];
+  __shared__ double tot[kKryPartials];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nv = 2 * (k + 1);
+  for (int q = threadIdx.x; q < nv * (kKryThreads / 32); q += kKryThreads) acc[q / (kKryThreads / 32)][q % (kKryThreads / 32)] = 0.0;
+  __syncthreads();
+  const long n2 = n >> 1;
+  const double2 *w2 = reinterpret_cast<const double2 *>(w);
+  const long tiles = (n2 + kKryTile - 1) / kKryTile;
+  for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const long q0 = tile * kKryTile + threadIdx.x;
+    bool in[kKryPieces];
+    double2 a[kKryPieces], b[kKryPieces], x[kKryPieces], y[kKryPieces];
+    auto load = [&](double2 (&v)[kKryPieces], const double *p) {
+      const double2 *p2 = reinterpret_cast<const double2 *>(p);
+#pragma unroll
+      for (int e = 0; e < kKryPieces; e++)
+        v[e] = in[e] ? __ldg(p2 + q0 + e * kKryThreads) : make_double2(0.0, 0.0);
+    };
+#pragma unroll
+    for (int e = 0; e < kKryPieces; e++) {
+      in[e] = q0 + e * kKryThreads < n2;
+      a[e] = in[e] ? w2[q0 + e * kKryThreads] : make_double2(0.0, 0.0);
+    }
+    load(b, V + (size_t)k * n);
+    auto fold = [&](const double2 (&v)[kKryPieces], int i) {
+      double d = 0.0, g = 0.0;
+#pragma unroll
+      for (int e = 0; e < kKryPieces; e++) {
+        d += a[e].x * v[e].x;
+        d += a[e].y * v[e].y;
+        g += b[e].x * v[e].x;
+        g += b[e].y * v[e].y;
+      }
+      const double keep = lane & 1 ? g : d, send = lane & 1 ? d : g;
+      double s = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+#pragma unroll
+      for (int o = 2; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane < 2) acc[2 * i + lane][warp] += s;
+    };
+    load(x, V);
+    for (int i = 0; i <= k; i += 2) {
+      if (i + 1 <= k) load(y, V + (size_t)(i + 1) * n);
+      fold(x, i);
+      if (i + 1 > k) break;
+      if (i + 2 <= k) load(x, V + (size_t)(i + 2) * n);
+      fold(y, i + 1);
+    }
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < nv; q += kKryThreads) {
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < kKryThreads / 32; c++) s += acc[q][c];
+    partial[(size_t)q * gridDim.x + blockIdx.x] = s;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(cnt, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int q = warp; q < nv; q += kKryThreads / 32) {
+    double s = 0.0;
+    for (int c = lane; c < (int)gridDim.x; c += 32) s += __ldcg(partial + (size_t)q * gridDim.x + c);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) tot[q] = s;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    // lane l holds columns l, l + 32 and l + 64; row i of G is used at step i
+    double c[3];
+#pragma unroll
+    for (int m = 0; m < 3; m++) c[m] = lane + 32 * m <= k ? tot[2 * (lane + 32 * m)] : 0.0;
+    for (int i = lane; i < k; i += 32) gram[i * kKryGramLd + k] = tot[2 * i + 1];
+    __syncwarp();
+    for (int i = 0; i < k; i++) {
+      const double ci = __shfl_sync(0xffffffffu, i < 32 ? c[0] : (i < 64 ? c[1] : c[2]), i & 31);
+#pragma unroll
+      for (int m = 0; m < 3; m++) {
+        const int j = lane + 32 * m;
+        if (j > i && j <= k) c[m] = c[m] - ci * gram[i * kKryGramLd + j];
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 3; m++)
+      if (lane + 32 * m <= k) h[lane + 32 * m] = c[m];
+    if (lane == 0) *cnt = 0;
+  }
+}
+
+static __global__ void __launch_bounds__(kKryThreads, 2)
+    k_kry_sub(double *__restrict__ w, const double *__restrict__ V, int k, long n, double *partial, unsigned *cnt,
+              double *h) {
+  __shared__ double sh[32], c[kKryGramLd];
+  for (int q = threadIdx.x; q <= k; q += kKryThreads) c[q] = h[q];
+  __syncthreads();
+  const long n2 = n >> 1;
+  double2 *w2 = reinterpret_cast<double2 *>(w);
+  const long tiles = (n2 + kKryTile - 1) / kKryTile;
+  double s = 0.0;
+  for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const long q0 = tile * kKryTile + threadIdx.x;
+    bool in[kKryPieces];
+    double2 a[kKryPieces], x[kKryPieces], y[kKryPieces];
+    auto load = [&](double2 (&v)[kKryPieces], const double *p) {
+      const double2 *p2 = reinterpret_cast<const double2 *>(p);
+#pragma unroll
+      for (int e = 0; e < kKryPieces; e++)
+        v[e] = in[e] ? __ldg(p2 + q0 + e * kKryThreads) : make_double2(0.0, 0.0);
+    };
+#pragma unroll
+    for (int e = 0; e < kKryPieces; e++) {
+      in[e] = q0 + e * kKryThreads < n2;
+      a[e] = in[e] ? w2[q0 + e * kKryThreads] : make_double2(0.0, 0.0);
+    }
+    auto sub = [&](const double2 (&v)[kKryPieces], double ci) {
+#pragma unroll
+      for (int e = 0; e < kKryPieces; e++) {
+        a[e].x = a[e].x - ci * v[e].x;
+        a[e].y = a[e].y - ci * v[e].y;
+      }
+    };
+    load(x, V);
+    for (int i = 0; i <= k; i += 2) {
+      if (i + 1 <= k) load(y, V + (size_t)(i + 1) * n);
+      sub(x, c[i]);
+      if (i + 1 > k) break;
+      if (i + 2 <= k) load(x, V + (size_t)(i + 2) * n);
+      sub(y, c[i + 1]);
+    }
+#pragma unroll
+    for (int e = 0; e < kKryPieces; e++) {
+      if (in[e]) w2[q0 + e * kKryThreads] = a[e];
+      s += a[e].x * a[e].x;
+      s += a[e].y * a[e].y;
+    }
+  }
+  kry_finish(s, partial, cnt, h + k + 1, sh);
+}
+
 // Orthogonalisation of w against the Krylov vectors V_0..V_k (V_q at
 // V + q n), the Hessenberg column into h[0..k+1] (h[k+1] = |w|^2 before the
 // normalisation), as modified Gram-Schmidt.  With the knob
 // kTuneKryGsSteps = 1, one pass per step (k_kry_mgs_t); with S = 2..4, one
 // pass per S steps (k_kry_gs), which reads 2S vectors and w and writes w per
 // S steps instead of 3S and S: the same coefficients in exact arithmetic,
-// rounded differently.  tmp: 18 device doubles; partial: 10 x kKryMaxBlocks.
-inline void kry_orth(double *w, const double *V, int k, long n, double *h, double *tmp, double *partial,
+// rounded differently.  S = kKryAllSteps: all steps in two passes
+// (k_kry_dots, k_kry_sub).  tmp: 18 device doubles; partial: kKryPartials x
+// kKryMaxBlocks; gram: kKryGramLd^2, kept from one column to the next.
+inline void kry_orth(double *w, const double *V, int k, long n, double *h, double *tmp, double *gram, double *partial,
                      unsigned *cnt, cudaStream_t st) {
+  if (tune_value(kTuneKryGsSteps) == kKryAllSteps) {
+    const int g = kry_pass_grid(n);
+    k_kry_dots<<<g, kKryThreads, 0, st>>>(w, V, k, n, partial, cnt, gram, h);
+    k_kry_sub<<<g, kKryThreads, 0, st>>>(w, V, k, n, partial, cnt, h);
+    return;
+  }
   if (tune_value(kTuneKryGsSteps) < 2) {
     for (int q = 0; q <= k + 1; q++) {
       const double *vq = q > 0 ? V + (size_t)(q - 1) * n : nullptr;
