@@ -739,7 +739,7 @@ int gmres(int &iError, cudaStream_t st) {
       if ((r = matvec(Vk, H.t, st))) return r;
       if ((r = precond(H.t, H.w, st))) return r;
       if (H.p.TypePrecond == BX_PRECOND_BILU && learned_collecting() && (r = collect_pair(H.t, H.w, st))) return r;
-      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, st);  // scal 160..177
+      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, tune_value(kTuneKryGsSteps), st);  // scal 160..177
       CKH(cudaGetLastError());
       CKH(cudaMemcpyAsync(hb.data(), hdev, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, st));
       CKH(cudaStreamSynchronize(st));
@@ -824,7 +824,7 @@ int fgmres(int &iError, cudaStream_t st) {
       double *Vk = Vb + (size_t)k * N, *Zk = Zb + (size_t)k * N;
       if ((r = precond(Vk, Zk, st))) return r;
       if ((r = matvec(Zk, H.w, st))) return r;
-      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, st);  // scal 160..177
+      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, tune_value(kTuneKryGsSteps), st);  // scal 160..177
       CKH(cudaGetLastError());
       CKH(cudaMemcpyAsync(hb.data(), hdev, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, st));
       CKH(cudaStreamSynchronize(st));

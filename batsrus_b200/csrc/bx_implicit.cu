@@ -127,6 +127,9 @@ int residual(const double *in, const TmaMaps &map, double *out, bool lowOrder) {
   a.dtCellIn = lowOrder ? I.dtCell : nullptr;
   a.dtCellOut = lowOrder ? nullptr : I.dtCell;
   a.dtScale = 0.5;
+  // a single-level grid: resolution-change code only for a limiter sharper at
+  // float sides than elsewhere
+  a.anySpecial = a.nOrder > 1 && a.betaRc < a.beta;
   const int flux = lowOrder && I.p.TypeFluxImpl >= 0 ? I.p.TypeFluxImpl : c.sch.TypeFlux;
   cudaError_t e = launch_stage3d(c.shape, flux, kKindFp64, map, a, c.nSM, c.st);
   if (e != cudaSuccess) return core_fail(BX_ERR_CUDA, "residual launch: %s", cudaGetErrorString(e));
@@ -214,6 +217,10 @@ int gmres(int &iError) {
   const double *rvec = I.Rhs;
   std::vector<double> H((m + 1) * m), cs(m), sn(m), gv(m + 1), hb(m + 2), y(m);
   double *hdev = I.scal + 8;  // h_0 .. h_{k+1}
+  // three Gram-Schmidt steps per pass unless the caller sets the knob: the
+  // finite differences of the products amplify a change of the rounding (the
+  // two-pass columns move single cells by up to 1e-6 of the state's norm)
+  const int steps = tune_knob(kTuneKryGsSteps).tuned == 2 ? tune_value(kTuneKryGsSteps) : 3;
   while (true) {
     k_kry_scale<<<kry_grid(), kKryThreads, 0, c.st>>>(I.V, rvec, I.scal + 2, 1, N);  // V0 = r/||r||
     CKI(cudaGetLastError());
@@ -226,7 +233,7 @@ int gmres(int &iError) {
       if ((r = precond(Vk, Zk))) return r;
       if (learned_collecting() && c.nI == 8 && (r = learned_collect(Vk, Zk, c.nBlock, c.st))) return r;
       if ((r = matvec(Zk, I.W))) return r;
-      kry_orth(I.W, I.V, k, N, hdev, I.scal + 104, I.gram, I.partial, I.cnt, c.st);  // scal 104..121
+      kry_orth(I.W, I.V, k, N, hdev, I.scal + 104, I.gram, I.partial, I.cnt, steps, c.st);  // scal 104..121
       CKI(cudaGetLastError());
       CKI(cudaMemcpyAsync(hb.data(), hdev, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, c.st));
       CKI(cudaStreamSynchronize(c.st));

@@ -495,22 +495,22 @@ static __global__ void __launch_bounds__(kKryThreads, 2)
 
 // Orthogonalisation of w against the Krylov vectors V_0..V_k (V_q at
 // V + q n), the Hessenberg column into h[0..k+1] (h[k+1] = |w|^2 before the
-// normalisation), as modified Gram-Schmidt.  With the knob
-// kTuneKryGsSteps = 1, one pass per step (k_kry_mgs_t); with S = 2..4, one
+// normalisation), as modified Gram-Schmidt.  With steps = 1 (the knob
+// kTuneKryGsSteps), one pass per step (k_kry_mgs_t); with S = 2..4, one
 // pass per S steps (k_kry_gs), which reads 2S vectors and w and writes w per
 // S steps instead of 3S and S: the same coefficients in exact arithmetic,
 // rounded differently.  S = kKryAllSteps: all steps in two passes
 // (k_kry_dots, k_kry_sub).  tmp: 18 device doubles; partial: kKryPartials x
 // kKryMaxBlocks; gram: kKryGramLd^2, kept from one column to the next.
 inline void kry_orth(double *w, const double *V, int k, long n, double *h, double *tmp, double *gram, double *partial,
-                     unsigned *cnt, cudaStream_t st) {
-  if (tune_value(kTuneKryGsSteps) == kKryAllSteps) {
+                     unsigned *cnt, int steps, cudaStream_t st) {
+  if (steps == kKryAllSteps) {
     const int g = kry_pass_grid(n);
     k_kry_dots<<<g, kKryThreads, 0, st>>>(w, V, k, n, partial, cnt, gram, h);
     k_kry_sub<<<g, kKryThreads, 0, st>>>(w, V, k, n, partial, cnt, h);
     return;
   }
-  if (tune_value(kTuneKryGsSteps) < 2) {
+  if (steps < 2) {
     for (int q = 0; q <= k + 1; q++) {
       const double *vq = q > 0 ? V + (size_t)(q - 1) * n : nullptr;
       const double *hq = q > 0 ? h + q - 1 : nullptr;
@@ -521,7 +521,7 @@ inline void kry_orth(double *w, const double *V, int k, long n, double *h, doubl
   }
   // groups of S vectors: a pass subtracts one group and takes the inner
   // products (and Gram entries) of the next; tmp holds two sets of 9
-  const int S = tune_value(kTuneKryGsSteps);
+  const int S = steps;
   auto count = [&](int q0) { return q0 > k ? 0 : (k + 1 - q0 < S ? k + 1 - q0 : S); };
   auto fill = [&](GsArgs &a, int q0, int nc, double *to, int slotNorm) {
     for (int j = 0; j < nc; j++) a.vc[j] = V + (size_t)(q0 + j) * n;

@@ -40,6 +40,17 @@ cudaError_t launch8_lim(const TmaMaps &maps, const StageArgs &a, int nSM, cudaSt
 }
 
 template <bool RC>
+cudaError_t launch8_residual(int flux, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
+  switch (flux) {
+    case kFluxRusanov: return launch8_lim<512, 1, double, double, double, kFluxRusanov, RC>(maps, a, nSM, st);
+    case kFluxLinde: return launch8_lim<512, 1, double, double, double, kFluxLinde, RC>(maps, a, nSM, st);
+    case kFluxHlld: return launch8_lim<512, 1, double, double, double, kFluxHlld, RC>(maps, a, nSM, st);
+    case kFluxRoe: return launch8_lim<512, 1, double, double, double, kFluxRoe, RC>(maps, a, nSM, st);
+  }
+  return cudaErrorInvalidValue;
+}
+
+template <bool RC>
 cudaError_t launch8_roe(int kind, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
   switch (kind) {
     case kKindFp64: return launch8_lim<512, 1, double, double, double, kFluxRoe, RC>(maps, a, nSM, st);
@@ -52,13 +63,8 @@ cudaError_t launch8_roe(int kind, const TmaMaps &maps, const StageArgs &a, int n
 }  // namespace
 
 cudaError_t launch_stage8_residual(int flux, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
-  switch (flux) {
-    case kFluxRusanov: return launch8_lim<512, 1, double, double, double, kFluxRusanov, true>(maps, a, nSM, st);
-    case kFluxLinde: return launch8_lim<512, 1, double, double, double, kFluxLinde, true>(maps, a, nSM, st);
-    case kFluxHlld: return launch8_lim<512, 1, double, double, double, kFluxHlld, true>(maps, a, nSM, st);
-    case kFluxRoe: return launch8_lim<512, 1, double, double, double, kFluxRoe, true>(maps, a, nSM, st);
-  }
-  return cudaErrorInvalidValue;
+  if (a.anySpecial) return launch8_residual<true>(flux, maps, a, nSM, st);
+  return launch8_residual<false>(flux, maps, a, nSM, st);
 }
 
 cudaError_t launch_stage8_roe(int kind, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {

@@ -18,7 +18,8 @@ enum TuneKnob {
   kTuneBiluThreads,    // JFNK BILU sweeps: threads per block CTA (8 per cell of a wavefront)
   kTuneStageVariant,   // stage kernel, 8^3 blocks: 0 and 3 units of 128 cells (bx_stage_unit.cuh); one
                        // direction at a time with 1: one face per thread (576 threads), 2: two (288)
-  kTuneKryGsSteps,     // Gram-Schmidt steps per pass over w (1 to 4, 64: all); set, not timed
+  kTuneKryGsSteps,     // Gram-Schmidt steps per pass over w (1 to 4, 64: all; implicit step: 3
+                       // unless set); set, not timed
   kNumTune
 };
 
