@@ -959,9 +959,7 @@ int copy_out(double *h, const double *d) {
 
 }  // namespace
 
-void bx::heat_release() {
-  if (H.ready) free_heat();
-}
+void bx::heat_release() { free_heat(); }
 
 // autotune the warps per CTA of the ILU sweeps on the current system
 int bx::tune_heat() {
@@ -1008,12 +1006,20 @@ int bx_heat_init(const bx_heat_params *prm, const double *Te, const double *bhat
     return core_fail(BX_ERR_ARG, "PrecondPrecision=%d", prm->PrecondPrecision);
   if (prm->OperatorPrecision != BX_FP64 && prm->OperatorPrecision != BX_FP32_BULK)
     return core_fail(BX_ERR_ARG, "OperatorPrecision=%d", prm->OperatorPrecision);
-  if (H.ready) free_heat();
+  // a new start on a grid of the same size keeps the buffers: allocating and
+  // freeing 40 vectors took longer than a solve at 128^3
+  const bool keep = H.ready && H.nBlock == c.nBlock && H.ilu32 == (prm->PrecondPrecision == BX_FP32_BULK) &&
+                    H.op32 == (prm->OperatorPrecision == BX_FP32_BULK) && H.p.nKrylovVector == prm->nKrylovVector;
+  if (!keep) free_heat();
+  H.ready = false;
   H.ilu32 = prm->PrecondPrecision == BX_FP32_BULK;
   H.op32 = prm->OperatorPrecision == BX_FP32_BULK;
   std::vector<int> atH, xyzH;
   const int r0 = grid_tables(c, atH, xyzH);
-  if (r0) return r0;
+  if (r0) {
+    free_heat();
+    return r0;
+  }
   H.p = *prm;
   H.nBlock = c.nBlock;
   H.nCell = (long)c.nBlock * kNC;
@@ -1033,27 +1039,29 @@ int bx_heat_init(const bx_heat_params *prm, const double *Te, const double *bhat
   H.a.sic = prm->SemiImplCoeff;
   const size_t vb = sizeof(double) * H.nCell;
   bool ok = true;
-  for (double **p : {&H.Te, &H.HC, &H.b, &H.x, &H.w, &H.t, &H.r}) ok = ok && cudaMalloc(p, vb) == cudaSuccess;
-  const size_t cfBytes = (H.ilu32 ? sizeof(float4) : sizeof(double4)) * H.nCell;
-  ok = ok && cudaMalloc(&H.B3, 3 * vb) == cudaSuccess &&
-       cudaMalloc(&H.coef, cfBytes) == cudaSuccess &&
-       cudaMalloc(&H.K, sizeof(double) * kKBlock * H.nBlock) == cudaSuccess &&
-       (!H.op32 || cudaMalloc(&H.K32, sizeof(float) * kKBlock * H.nBlock) == cudaSuccess) &&
-       cudaMalloc(&H.wtab, sizeof(WaveTable)) == cudaSuccess && cudaMalloc(&H.cnt, sizeof(unsigned)) == cudaSuccess &&
-       cudaMalloc(&H.errDev, sizeof(int)) == cudaSuccess &&
-       cudaMalloc(&H.V, vb * (prm->nKrylovVector + 1)) == cudaSuccess &&
-       cudaMalloc(&H.used, H.nCell) == cudaSuccess &&
-       cudaMalloc(&H.blkAt, sizeof(int) * atH.size()) == cudaSuccess &&
-       cudaMalloc(&H.blkXYZ, sizeof(int) * xyzH.size()) == cudaSuccess &&
-       cudaMalloc(&H.partial, sizeof(double) * kKryPartials * kKryMaxBlocks) == cudaSuccess &&
-       cudaMalloc(&H.gram, sizeof(double) * kKryGramLd * kKryGramLd) == cudaSuccess &&
-       cudaMalloc(&H.scal, sizeof(double) * 192) == cudaSuccess;
+  if (!keep) {
+    for (double **p : {&H.Te, &H.HC, &H.b, &H.x, &H.w, &H.t, &H.r}) ok = ok && cudaMalloc(p, vb) == cudaSuccess;
+    const size_t cfBytes = (H.ilu32 ? sizeof(float4) : sizeof(double4)) * H.nCell;
+    ok = ok && cudaMalloc(&H.B3, 3 * vb) == cudaSuccess &&
+         cudaMalloc(&H.coef, cfBytes) == cudaSuccess &&
+         cudaMalloc(&H.K, sizeof(double) * kKBlock * H.nBlock) == cudaSuccess &&
+         (!H.op32 || cudaMalloc(&H.K32, sizeof(float) * kKBlock * H.nBlock) == cudaSuccess) &&
+         cudaMalloc(&H.wtab, sizeof(WaveTable)) == cudaSuccess && cudaMalloc(&H.cnt, sizeof(unsigned)) == cudaSuccess &&
+         cudaMalloc(&H.errDev, sizeof(int)) == cudaSuccess &&
+         cudaMalloc(&H.V, vb * (prm->nKrylovVector + 1)) == cudaSuccess &&
+         cudaMalloc(&H.used, H.nCell) == cudaSuccess &&
+         cudaMalloc(&H.blkAt, sizeof(int) * atH.size()) == cudaSuccess &&
+         cudaMalloc(&H.blkXYZ, sizeof(int) * xyzH.size()) == cudaSuccess &&
+         cudaMalloc(&H.partial, sizeof(double) * kKryPartials * kKryMaxBlocks) == cudaSuccess &&
+         cudaMalloc(&H.gram, sizeof(double) * kKryGramLd * kKryGramLd) == cudaSuccess &&
+         cudaMalloc(&H.scal, sizeof(double) * 192) == cudaSuccess;
+  }
   if (!ok) {
     free_heat();
     return core_fail(BX_ERR_NOMEM, "heat conduction buffers");
   }
-  CKH(cudaEventCreate(&H.ev[0]));
-  CKH(cudaEventCreate(&H.ev[1]));
+  for (auto &e : H.ev)
+    if (!e) CKH(cudaEventCreate(&e));
   CKH(cudaMemcpyAsync(H.Te, Te, vb, cudaMemcpyHostToDevice, c.st));
   CKH(cudaMemcpyAsync(H.B3, bhat, 3 * vb, cudaMemcpyHostToDevice, c.st));
   CKH(cudaMemcpyAsync(H.used, used, H.nCell, cudaMemcpyHostToDevice, c.st));
