@@ -215,6 +215,19 @@ __global__ void k_collect_mc(const double4 *__restrict__ coefL, const unsigned c
                   (uc && j > 0 && u[c - 8]) ? (float)v.y : 0.f, (uc && k > 0 && u[c - 64]) ? (float)v.z : 0.f);
 }
 
+// n floats (a multiple of 8) rounded to BF16, 32 bytes in and 16 out per thread
+__global__ void k_to_bf16(const float *__restrict__ x, __nv_bfloat16 *__restrict__ y, long n) {
+  for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n / 8; q += (long)gridDim.x * blockDim.x) {
+    const float4 a = reinterpret_cast<const float4 *>(x)[2 * q], b = reinterpret_cast<const float4 *>(x)[2 * q + 1];
+    uint4 o;
+    o.x = pack_bf16x2(a.x, a.y);
+    o.y = pack_bf16x2(a.z, a.w);
+    o.z = pack_bf16x2(b.x, b.y);
+    o.w = pack_bf16x2(b.z, b.w);
+    reinterpret_cast<uint4 *>(y)[q] = o;
+  }
+}
+
 // out[0] += sum tgt . x, out[1] += sum x . x over cells [0, nCell) (x = the
 // first 8 input channels)
 __global__ void k_ident_fit(const __nv_bfloat16 *__restrict__ in16, const float *__restrict__ tgt, long nCell,
@@ -535,9 +548,16 @@ int bx_learned_set_samples(const float *in16, const float *tgt, long long nSampl
   if (r) return r;
   if (!in16 || !tgt || nSample < 1 || nSample > Lc.nSampleMax)
     return core_fail(BX_ERR_ARG, "nSample=%lld outside 1..%ld", nSample, Lc.nSampleMax);
-  std::vector<__nv_bfloat16> h((size_t)nSample * 512 * 16);
-  for (size_t i = 0; i < h.size(); i++) h[i] = __float2bfloat16_rn(in16[i]);
-  CKL(cudaMemcpyAsync(Lc.in16, h.data(), sizeof(__nv_bfloat16) * h.size(), cudaMemcpyHostToDevice, Lc.st));
+  // rounded to BF16 on the device, a piece at a time through the activation
+  // buffers (idle here): 8.4 M numbers took 12 ms on the host
+  const long n = nSample * 512 * 16, piece = (long)kBatchMax * 512 * 32 / 2;  // floats that A1 holds
+  for (long o = 0, q = 0; o < n; o += piece, q++) {
+    const long m = std::min(piece, n - o);
+    float *buf = reinterpret_cast<float *>(q & 1 ? Lc.A2 : Lc.A1);
+    CKL(cudaMemcpyAsync(buf, in16 + o, sizeof(float) * m, cudaMemcpyHostToDevice, Lc.st));
+    k_to_bf16<<<4 * Lc.nSM, 256, 0, Lc.st>>>(buf, Lc.in16 + o, m);
+    CKL(cudaGetLastError());
+  }
   CKL(cudaMemcpyAsync(Lc.tgt, tgt, sizeof(float) * 512 * 8 * (size_t)nSample, cudaMemcpyHostToDevice, Lc.st));
   CKL(cudaStreamSynchronize(Lc.st));
   Lc.nSample = nSample;
