@@ -1,7 +1,7 @@
 """Build libbx200.so in-tree with nvcc for sm_100a.
 
-The FP64 stage kernels and the per-block kernels are compiled with
---fmad=false: the reference's arithmetic is not contracted into fused
+The 1D stage kernel, the per-block kernels and the implicit step's vector
+kernels are compiled with --fmad=false: the reference's arithmetic is not contracted into fused
 multiply-adds, so the GPU FP64 path keeps the reference operation order.
 """
 import os
@@ -21,6 +21,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 # (source, extra flags)
 UNITS = [
     ("bx_compat.cu", ["--fmad=false"]),
+    ("bx_stage_line.cu", ["--fmad=false"]),
     ("bx_stage_flat.cu", []),
     ("bx_stage3d.cu", []),
     ("bx_stage3d_fpt2.cu", []),
@@ -38,7 +39,7 @@ UNITS = [
     ("bx_tune.cu", []),
     ("bx_capi.cu", []),
 ]
-HEADERS = ["bx_physics.cuh", "bx_stage.cuh", "bx_device.h", "bx_stage3d.cuh", "bx_stage3d_v2.cuh", "bx_stage3d_launch.cuh", "bx_stage_unit.cuh", "bx_stage_flat.cuh",
+HEADERS = ["bx_physics.cuh", "bx_stage.cuh", "bx_device.h", "bx_stage3d.cuh", "bx_stage3d_v2.cuh", "bx_stage3d_launch.cuh", "bx_stage_unit.cuh", "bx_stage_flat.cuh", "bx_stage_line.cuh",
            "bx_stage_unit_launch.cuh", "bx_tma.cuh", "bx_core.h",
            "bx_impl_kernels.cuh", "bx_krylov.cuh", "bx_tune.h", "bx_tc.cuh", "bx_learned.cuh", "bx_learned_kernels.cuh", "bx_amr.h"]
 

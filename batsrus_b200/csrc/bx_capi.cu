@@ -390,7 +390,8 @@ int launch_stage_dt(int iStage, bool computeDt, int finish = 0, double tLimit = 
     }
     e = launch_stage3d(g.shape, g.sch.TypeFlux, kind, *m, a, g.nSM, g.st);
   } else {
-    e = launch_stage_flat(g.shape, g.sch.TypeFlux, a, g.st);
+    e = g.shape == kShape881 ? launch_stage_flat(g.sch.TypeFlux, a, g.st)
+                             : launch_stage_line(g.shape, g.sch.TypeFlux, a, g.st);
   }
   if (e != cudaSuccess) return fail(BX_ERR_CUDA, "stage kernel launch: %s", cudaGetErrorString(e));
   if (g.timing) { CK(cudaEventRecord(g.evStop[g.nTimed], g.st)); g.nTimed++; }
