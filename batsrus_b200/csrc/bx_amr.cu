@@ -34,6 +34,10 @@ __device__ __forceinline__ long gidx(const int *lc, int blk, int e, int N, int x
   return (long)lc[4 * blk + 1 + e] * N + x;
 }
 
+// a global cell index at most one period outside [0, tot), wrapped (a 64-bit
+// remainder costs more than the loads of a ghost cell)
+__device__ __forceinline__ long wrap1(long x, long tot) { return x < 0 ? x + tot : (x >= tot ? x - tot : x); }
+
 // state value (variable v) of the ghost cell x3 (block-local coordinates,
 // x3[d] = -1 - l or N + l) across the resolution-change side S, as
 // exchange_messages leaves it: a coarser neighbour's cell copied into the
@@ -54,8 +58,7 @@ __device__ __forceinline__ double rc_ghost_value(const InT *in, const RcSlab &S,
     int c3[3];
     for (int e = 0; e < 3; e++) {
       const long tot = (long)N * ((long)nr[e] << lev);
-      long gf = gidx(lc, S.block, e, N, x3[e]);
-      gf = (gf + tot) % tot;
+      const long gf = wrap1(gidx(lc, S.block, e, N, x3[e]), tot);
       c3[e] = (int)((gf >> 1) - (long)lc[4 * C + 1 + e] * N);
     }
     if (twoLayers && (hi ? x3[d] - N : -1 - x3[d]) == 1) c3[d] += hi ? 1 : -1;
@@ -66,7 +69,7 @@ __device__ __forceinline__ double rc_ghost_value(const InT *in, const RcSlab &S,
   long f0[3];
   for (int e = 0; e < 3; e++) {
     const long tot = (long)N * ((long)nr[e] << lev);
-    const long gc = (gidx(lc, S.block, e, N, x3[e]) + tot) % tot;
+    const long gc = wrap1(gidx(lc, S.block, e, N, x3[e]), tot);
     f0[e] = 2 * gc - (long)lc[4 * F + 1 + e] * N;
   }
   f0[d] += hi ? 0 : 1;

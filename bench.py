@@ -49,16 +49,14 @@ def peaks():
 
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell of one
-# stage8_kernel launch, the mean of a stage-1 and a stage-2 launch, from ncu
-# captures of the 160^3 Orszag-Tang case (20^3 blocks, 0.26 GB of state,
-# larger than L2):
-#   python bench.py --nroot 20 --precisions <p> --steps 2 --warmup 3 --no-e2e --no-cpu \
-#       --no-amr --jfnk-precond= --heat-precond= --no-autotune
-#   ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum \
-#       --clock-control none -k regex:stage8 -s 2 -c 2 --csv <same command>
-# FP64: 135.8 and 200.1 B; FP32-bulk: 111.8 and 159.0 B.  Traffic grows in
+# stage_unit_kernel launch, the mean of a stage-1 and a stage-2 launch, from
+# ncu captures of three steps of the 160^3 Orszag-Tang case (20^3 blocks, 0.26
+# GB of state, larger than L2), --metrics
+# gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum
+# --clock-control none -k regex:stage_unit.
+# FP64: 136.9 and 202.1 B; FP32-bulk: 106.8 and 157.2 B.  Traffic grows in
 # proportion to the blocks, so the bench scales it by the cells of its grid.
-DRAM_BYTES_PER_CELL_LAUNCH = {"fp64": 168.0, "fp32": 135.4}
+DRAM_BYTES_PER_CELL_LAUNCH = {"fp64": 169.5, "fp32": 132.0}
 
 
 def profile_traffic(prec):
@@ -190,7 +188,8 @@ def run_ours(args):
                             "unit": "GB/s", "frac": round(achieved / hbm_peak, 4),
                             "traffic": (t_per_cell * nCell if t_per_cell else None),
                             "peak_source": peak_kind},
-               "clocks": clk.summary(), "gpu_launches": 4 * args.steps,
+               "clocks": clk.summary(), # two stage launches per step and the first step's time step (Roe: two bookkeeping launches more)
+               "gpu_launches": 4 * args.steps if args.flux == "Roe" else 2 * args.steps + 1,
                "autotune": ({k: v["value"] for k, v in tuned.items()} if tuned else None)}
         # ---- end to end through the C ABI with pinned host buffers ----------
         if args.e2e:
@@ -680,7 +679,7 @@ def main():
     ap.add_argument("--sharded", action="store_true",
                     help="one domain partitioned over the ranks (shard.GpuRank) instead of replicas")
     ap.add_argument("--stage-ctas", type=int, default=0,
-                    help="pin stage_ctas_per_sm (FP32-bulk stage 2: 2 -> two 256-thread CTAs per SM)")
+                    help="pin stage_ctas_per_sm (at most this many CTAs of the stage kernel per SM)")
     ap.add_argument("--no-autotune", dest="autotune", action="store_false",
                     help="keep the default launch shapes instead of bx_autotune")
     ap.add_argument("--heat-precond", default="BILU,NONE,LEARNED", help="'' to skip the heat conduction workload")
