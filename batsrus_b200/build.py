@@ -1,6 +1,6 @@
 """Build libbx200.so in-tree with nvcc for sm_100a.
 
-The 1D stage kernel, the per-block kernels and the implicit step's vector
+The 1D and 2D stage kernels, the per-block kernels and the implicit step's vector
 kernels are compiled with --fmad=false: the reference's arithmetic is not contracted into fused
 multiply-adds, so the GPU FP64 path keeps the reference operation order.
 """
@@ -22,7 +22,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 UNITS = [
     ("bx_compat.cu", ["--fmad=false"]),
     ("bx_stage_line.cu", ["--fmad=false"]),
-    ("bx_stage_flat.cu", []),
+    ("bx_stage_flat.cu", ["--fmad=false"]),
     ("bx_stage3d.cu", []),
     ("bx_stage3d_fpt2.cu", []),
     ("bx_stage3d_v2.cu", []),

@@ -124,7 +124,7 @@ struct StageArgs {
 };
 
 #ifdef __CUDACC__
-// The 1D and 2D stage kernel is launched as a programmatic dependent of the
+// The 1D stage kernel is launched as a programmatic dependent of the
 // kernel before it (launch_dependent): its CTAs may start, and load what no
 // kernel writes, while that kernel's last CTAs run; grid_wait returns when it
 // has ended and its writes are visible.  grid_go lets the next kernel start

@@ -1,188 +1,183 @@
-// bx_stage_flat.cuh -- fused explicit stage kernel of 2D blocks (FP64).
+// bx_stage_flat.cuh -- fused explicit stage kernel of 2D blocks (FP64): one CTA
+// per block, one sweep per direction.
 //
-// A CTA of one thread per face (five warps for the 144 faces of an 8 x 8
-// block) works through blocks; per block:
-//   1. gather: the block's cells and two ghost layers per side come straight
-//      from the neighbours' interiors (float boundaries copy the boundary
-//      cell), one cell per thread, loaded behind the faces of the block
-//      before, into a primitive tile in shared memory;
-//   2. faces: every face of both directions, one per thread, in the face's own
-//      frame (flux_frame, hlld_frame; bx_physics.cuh), into the slot buffer;
-//   3. cells: flux differences, Powell source, update and cell time step
-//      (update_cell).
-// Reference behaviour: update_state_fast (src/ModUpdateStateFast.f90:190)
-// and the orig path calc_face_value -> calc_face_flux -> calc_source ->
-// update_state (src/ModAdvanceExplicit.f90:140-226).
-//
-// What bounds it: the latency of the chain load - faces - update of a block
-// with 20 warps per SM (96 registers).  384 x 384 Linde + Koren per step, two
-// stages: 39.4 us; a CTA per block without the loads ahead 41.3; the kernel
-// before (255 registers, two sweeps, IEEE divisions) 87.
+// The arithmetic is the reference's, operation by operation (numerical_flux,
+// IEEE divisions and square roots, no contraction: compiled with
+// --fmad=false).  Runs with the minmod limiter amplify the rounding of a step
+// in 2D: the flux functions of the 3D kernel, with a thread per face and 20
+// warps per SM, took 39 us per step at 384 x 384 where the kernel before took 87,
+// but gave digits up to 2e-14 of the norm apart after 50 steps.  Kept of that
+// are five CTAs per SM (128 registers instead of 255) and the end of the time
+// step in the last CTA.  The gather loads through the read-only path, so the
+// kernel does not start before the one that writes the state has ended.
 #pragma once
-#include "bx_stage_unit.cuh"
+#include "bx_stage.cuh"
 
 namespace bx {
 
-template <int NI_, int NJ_>
-struct Flat {
-  static constexpr int NI = NI_, NJ = NJ_, NDIM = NJ > 1 ? 2 : 1, NC = NI * NJ;
-  // primitive tile: interior, x ghosts [row][4], y ghosts [4][i]
-  static constexpr int oX = NC, oY = oX + 4 * NJ, PT = oY + (NDIM > 1 ? 4 * NI : 0);
-  // faces: x faces n < NI of all rows, then the n = NI ones; y faces
-  static constexpr int F0 = (NI + 1) * NJ, F1 = NDIM > 1 ? NI * (NJ + 1) : 0, NF = F0 + F1;
-  static constexpr int NTHR = (NF + 31) / 32 * 32;
-  // CTAs per SM that the registers are limited for: 96 registers for a 2D block, but 128 for
-  // the Roe flux (630 bytes of spills with 96)
-  static constexpr int minb(int flux) { return NTHR > 96 ? (flux == kFluxRoe ? 3 : 4) : (NTHR > 32 ? 5 : 16); }
+// per-cell accumulators held in registers across the three sweeps
+struct CellAcc {
+  double chg[8];    // flux divergence sum (rho, m, B, E)
+  double divBint;   // DivBInternal_C
+  double dbf[6];    // dB1nFace1..6
+  double vdt;       // sum over dims of max(Vdt_left, Vdt_right)
 };
 
-template <class S, int FLUX, int LIM>
-__global__ void __launch_bounds__(S::NTHR, S::minb(FLUX)) stage_flat_kernel(const StageArgs a) {
-  constexpr int NI = S::NI, NJ = S::NJ, NC = S::NC, PT = S::PT, NF = S::NF;
-  __shared__ double P[8 * PT], fb[10 * NF], wmin[S::NTHR / 32];
-  // the owned blocks come first, so a CTA's blocks need no look-up (nor does
-  // the order matter: a 1D or 2D state lies in L2)
-  static_assert(PT <= S::NTHR, "one cell of the tile per thread");
-  const int t = threadIdx.x;
-  const double *in = reinterpret_cast<const double *>(a.in);
-  // the thread's cell of the tile, and the side it is a ghost cell of
-  int ci = 0, cj = 0, side = -1;
-  if (t < S::oX) {
-    ci = t % NI; cj = t / NI;
-  } else if (t < S::oY) {
-    const int g = (t - S::oX) & 3;
-    cj = (t - S::oX) >> 2;
-    ci = g < 2 ? g - 2 : NI + g - 2;
-    side = g < 2 ? 0 : 1;
-  } else if (t < PT) {
-    const int g = (t - S::oY) / NI;
-    ci = (t - S::oY) % NI;
-    cj = g < 2 ? g - 2 : NJ + g - 2;
-    side = g < 2 ? 2 : 3;
+template <class S, int D, int FLUX, typename Real>
+__device__ __forceinline__ void sweep(const StageArgs &a, const BlockGeom &g, const Real *tile,
+                                      Real *fbuf, CellAcc (&acc)[S::CPT], int &err) {
+  constexpr int NF = D == 0 ? S::NFX : (D == 1 ? S::NFY : S::NFZ);
+  const Real gamma = (Real)a.gamma, invGm1 = (Real)a.invGm1, beta = (Real)a.beta;
+  const Real area = (Real)g.area[D];
+  for (int f = threadIdx.x; f < NF; f += blockDim.x) {
+    int i, j, k;
+    face_decode<S, D>(f, i, j, k);
+    Real L[8], R[8], F[8], vdt;
+    face_states<S, D>(tile, i, j, k, a.nOrder, a.limiter, beta, L, R);
+    if (FLUX == kFluxRoe) {
+      // UseRS7 (src/ModFaceFlux.f90:600-625): each face state takes the
+      // normal field of its cell before the div B slots are formed; the
+      // Roe dissipation also uses the cells' normal velocities
+      constexpr int st = D == 0 ? 1 : (D == 1 ? S::TX : S::TX * S::TY);
+      const int c = S::t(i, j, k);
+      const Real cbL = tile[(kBx + D) * S::NT + c - st], cbR = tile[(kBx + D) * S::NT + c];
+      const Real cuL = tile[(kUx + D) * S::NT + c - st], cuR = tile[(kUx + D) * S::NT + c];
+      const Real dBnR = R[kBx + D] - cbR;
+      R[kBx + D] = R[kBx + D] - dBnR;
+      const Real dBnL = L[kBx + D] - cbL;
+      L[kBx + D] = L[kBx + D] - dBnL;
+      fbuf[9 * S::NFMAX + f] = L[kBx + D];
+      fbuf[10 * S::NFMAX + f] = R[kBx + D];
+      vdt = roe_flux<D>(L, R, cuL, cuR, dBnL, dBnR, gamma, invGm1, area, F, 1);
+    } else {
+      fbuf[9 * S::NFMAX + f] = L[kBx + D];
+      fbuf[10 * S::NFMAX + f] = R[kBx + D];
+      if (!numerical_flux<D, FLUX>(L, R, gamma, invGm1, area, F, vdt)) err = 1;
+    }
+#pragma unroll
+    for (int v = 0; v < 8; v++) fbuf[v * S::NFMAX + f] = F[v];
+    fbuf[8 * S::NFMAX + f] = vdt;
   }
-  // its source in the neighbour across the side, or (float boundary) the
-  // boundary cell
-  const int cw = min(max(ci, 0), NI - 1) + NI * min(max(cj, 0), NJ - 1);
-  const int cn = (ci + NI) % NI + NI * ((cj + NJ) % NJ);
-  auto neighbour = [&](int b) { return side >= 0 && b < a.nBlock ? a.nbr[6 * b + side] : b; };
-  auto load = [&](int b, int nb, double (&w)[8]) {
-    const double *u = in + (size_t)(nb >= 0 ? nb : b) * 8 * NC + (nb >= 0 ? cn : cw);
+  __syncthreads();
+  const double h = g.invHalf[D];  // DxInvHalf = 0.5/CellSize
 #pragma unroll
-    for (int v = 0; v < 8; v++) w[v] = u[v * NC];
-  };
-  int nb = neighbour(blockIdx.x);
-  grid_go();
-  grid_wait();  // the neighbour table is constant; the state and the time step are the previous kernel's
-  const double DtNoCfl = a.ts->DtNoCfl;
-  double w[8];
-  if (t < PT) load(blockIdx.x, nb, w);
-
-  for (int b = blockIdx.x; b < a.nBlock; b += gridDim.x) {
-    if (t < PT) {
-      const double rhoInv = rcp_cell(w[kRho]);
-      w[kUx] = rhoInv * w[kUx];
-      w[kUy] = rhoInv * w[kUy];
-      w[kUz] = rhoInv * w[kUz];
+  for (int m = 0; m < S::CPT; m++) {
+    const int c = threadIdx.x + m * S::NTHREAD;
+    if (c < S::NC) {
+      const int i = c % S::NI, j = (c / S::NI) % S::NJ, k = c / (S::NI * S::NJ);
+      const int f0 = face_index<S, D>(i, j, k);
+      const int f1 = face_index<S, D>(i + (D == 0), j + (D == 1), k + (D == 2));
 #pragma unroll
-      for (int v = 0; v < 8; v++) P[t + v * PT] = w[v];
+      for (int v = 0; v < 8; v++) {
+        const double F0 = (double)fbuf[v * S::NFMAX + f0], F1 = (double)fbuf[v * S::NFMAX + f1];
+        acc[m].chg[v] = D == 0 ? F0 - F1 : acc[m].chg[v] + F0 - F1;
+      }
+      const double L0 = (double)fbuf[9 * S::NFMAX + f0], R0 = (double)fbuf[10 * S::NFMAX + f0];
+      const double L1 = (double)fbuf[9 * S::NFMAX + f1], R1 = (double)fbuf[10 * S::NFMAX + f1];
+      // calc_divb_source (src/ModCalcSource.f90:1694-1891)
+      const double inner = 2 * h * (L1 - R0);
+      acc[m].divBint = D == 0 ? inner : acc[m].divBint + inner;
+      acc[m].dbf[2 * D] = h * (R0 - L0);
+      acc[m].dbf[2 * D + 1] = h * (R1 - L1);
+      const double vmax = fmax((double)fbuf[8 * S::NFMAX + f0], (double)fbuf[8 * S::NFMAX + f1]);
+      acc[m].vdt = D == 0 ? vmax : acc[m].vdt + vmax;
     }
-    // the next block's neighbour now, its cells behind this block's faces
-    const int bn1 = b + gridDim.x;
-    nb = neighbour(bn1);
-    const BlockGeom g = a.geom[b];
+  }
+  __syncthreads();
+}
+
+template <class S, typename Real, typename InT, typename OutT, int FLUX>
+__global__ void __launch_bounds__(S::NTHREAD, 5) stage_flat_kernel(const StageArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Real *tile = reinterpret_cast<Real *>(smem_raw);
+  Real *fbuf = tile + 8 * S::NT;
+  __shared__ double wmin[32];
+
+  const int b = a.order[blockIdx.x];
+  int nb[6];
+#pragma unroll
+  for (int q = 0; q < 6; q++) nb[q] = a.nbr[6 * b + q];
+  const BlockGeom g = a.geom[b];
+
+  gather_tile<S, Real, InT>(reinterpret_cast<const InT *>(a.in), nb, b, tile);
+  __syncthreads();
+
+  CellAcc acc[S::CPT];
+  int err = 0;
+  sweep<S, 0, FLUX, Real>(a, g, tile, fbuf, acc, err);
+  if (S::NDIM > 1) sweep<S, 1, FLUX, Real>(a, g, tile, fbuf, acc, err);
+  if (S::NDIM > 2) sweep<S, 2, FLUX, Real>(a, g, tile, fbuf, acc, err);
+  if (err) atomicOr(&a.ts->errFlag, kErrHlld);
+
+  // ---- update (update_state_normal + update_explicit) --------------------
+  const StepState &ts = *a.ts;
+  const double DtNoCfl = ts.DtNoCfl;
+  const double DtFactor = a.useHalfStep ? (a.cfl * a.iStage) / a.nStage : a.cfl;
+  const double DtLocal = DtFactor * DtNoCfl;
+  const double invGm1 = a.invGm1, gm1 = a.gamma - 1.0;
+  const double V = g.volume;
+  double dtmin = 1e300;
+  const double *__restrict__ old = a.old + (size_t)b * 8 * S::NC;
+  OutT *__restrict__ out = reinterpret_cast<OutT *>(a.out) + (size_t)b * 8 * S::NC;
+#pragma unroll
+  for (int m = 0; m < S::CPT; m++) {
+    const int c = threadIdx.x + m * S::NTHREAD;
+    if (c >= S::NC) continue;
+    double o[8];
+#pragma unroll
+    for (int v = 0; v < 8; v++) o[v] = old[v * S::NC + c];
+    if (a.computeDt) dtmin = fmin(dtmin, V / acc[m].vdt);
+    if (DtNoCfl == 0.0) {  // IsTimeAccurate .and. Dt == 0: state unchanged, floored
+      o[kP] = limit_pressure(o[kRho], o[kP], a.fl.pMin, a.fl.tMin, a.fl.massIon);
+#pragma unroll
+      for (int v = 0; v < 8; v++) out[v * S::NC + c] = (OutT)o[v];
+      continue;
+    }
+    double src[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (a.useDivb) {
+      double divB = acc[m].divBint + acc[m].dbf[0] + acc[m].dbf[1];
+      if (S::NDIM > 1) divB = divB + acc[m].dbf[2] + acc[m].dbf[3];
+      if (S::NDIM > 2) divB = divB + acc[m].dbf[4] + acc[m].dbf[5];
+      const int i = c % S::NI, j = (c / S::NI) % S::NJ, k = c / (S::NI * S::NJ);
+      const int tt = S::t(i, j, k);
+      const double ux = tile[kUx * S::NT + tt], uy = tile[kUy * S::NT + tt], uz = tile[kUz * S::NT + tt];
+      const double bx = tile[kBx * S::NT + tt], by = tile[kBy * S::NT + tt], bz = tile[kBz * S::NT + tt];
+      src[kBx] = 0 - divB * ux; src[kBy] = 0 - divB * uy; src[kBz] = 0 - divB * uz;
+      src[kE] = 0 - divB * (bx * ux + by * uy + bz * uz);
+      src[kUx] = 0 + (0 - divB * bx); src[kUy] = 0 + (0 - divB * by); src[kUz] = 0 + (0 - divB * bz);
+    }
+    double s[8];
+#pragma unroll
+    for (int v = 0; v < 8; v++) s[v] = DtLocal * (src[v] + acc[m].chg[v] / V);
+    // pressure_to_energy(StateOld) (src/ModEnergy.f90:47)
+    double e = invGm1 * o[kP] + 0.5 * (o[kUx] * o[kUx] + o[kUy] * o[kUy] + o[kUz] * o[kUz]) / o[kRho];
+    e = e + 0.5 * (o[kBx] * o[kBx] + o[kBy] * o[kBy] + o[kBz] * o[kBz]);
+    double n[8];
+#pragma unroll
+    for (int v = 0; v < 7; v++) n[v] = o[v] + s[v];
+    e = e + s[kE];
+    if (a.fl.rhoMin > 0.0) n[kRho] = fmax(a.fl.rhoMin, n[kRho]);  // UseRhoMin
+    // energy_to_pressure (src/ModEnergy.f90:243), then limit_pressure
+    double p = e - 0.5 * (n[kBx] * n[kBx] + n[kBy] * n[kBy] + n[kBz] * n[kBz]);
+    n[kP] = gm1 * (p - 0.5 * (n[kUx] * n[kUx] + n[kUy] * n[kUy] + n[kUz] * n[kUz]) / n[kRho]);
+    n[kP] = limit_pressure(n[kRho], n[kP], a.fl.pMin, a.fl.tMin, a.fl.massIon);
+#pragma unroll
+    for (int v = 0; v < 8; v++) out[v * S::NC + c] = (OutT)n[v];
+  }
+
+  if (a.computeDt) {
+    // block minimum (calc_block_dt) then grid minimum (MPI_MIN of
+    // set_global_timestep) via atomicMin on the ordered bits
+    for (int off = 16; off > 0; off >>= 1) dtmin = fmin(dtmin, __shfl_xor_sync(0xffffffffu, dtmin, off));
+    if ((threadIdx.x & 31) == 0) wmin[threadIdx.x >> 5] = dtmin;
     __syncthreads();
-    if (t < PT && bn1 < a.nBlock) load(bn1, nb, w);
-
-    int err = 0;
-    if (t < NF) {
-      const int D = S::NDIM > 1 && t >= S::F0 ? 1 : 0;
-      int n, in0, sIn, gh, sGh, extent;
-      if (D == 0) {
-        const int row = t < NI * NJ ? t / NI : t - NI * NJ;
-        n = t < NI * NJ ? t % NI : NI;
-        in0 = row * NI; sIn = 1;
-        gh = S::oX + row * 4; sGh = 1;
-        extent = NI;
-      } else {
-        const int f = t - S::F0;
-        n = f / NI;
-        in0 = f % NI; sIn = NI;
-        gh = S::oY + in0; sGh = NI;
-        extent = NJ;
-      }
-      int ad[4];
-#pragma unroll
-      for (int m = 0; m < 4; m++) {
-        const int c = n - 2 + m;
-        ad[m] = (unsigned)c < (unsigned)extent ? in0 + c * sIn : gh + (c < 0 ? c + 2 : c - extent + 2) * sGh;
-      }
-      const int T1 = D + 1, T2 = D == 0 ? 2 : 0;
-      const int var[8] = {0, 1 + D, 1 + T1, 1 + T2, 4 + D, 4 + T1, 4 + T2, 7};
-      double L[8], R[8];
-      if (a.nOrder == 1) {
-#pragma unroll
-        for (int v = 0; v < 8; v++) { L[v] = P[ad[1] + var[v] * PT]; R[v] = P[ad[2] + var[v] * PT]; }
-      } else {
-#pragma unroll
-        for (int v = 0; v < 8; v++)
-          limited_face_t<LIM>(a.beta, P[ad[0] + var[v] * PT], P[ad[1] + var[v] * PT], P[ad[2] + var[v] * PT],
-                              P[ad[3] + var[v] * PT], L[v], R[v]);
-      }
-      double cbL = 0, cbR = 0, cuL = 0, cuR = 0, bn;
-      if (FLUX == kFluxRoe) {
-        cbL = P[ad[1] + var[4] * PT]; cbR = P[ad[2] + var[4] * PT];
-        cuL = P[ad[1] + var[1] * PT]; cuR = P[ad[2] + var[1] * PT];
-      }
-      bool ok = true;
-      const double vdt = unit_flux<FLUX, double>(D, L, R, a.gamma, a.invGm1, D == 0 ? g.area[0] : g.area[1], cbL, cbR, cuL, cuR, bn, ok,
-                                                 [&](int q, double x) { fb[var[q] * NF + t] = x; });
-      fb[8 * NF + t] = vdt;
-      fb[9 * NF + t] = bn;
-      if (!ok) err = 1;
+    if (threadIdx.x == 0) {
+      double m = wmin[0];
+      for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmin(m, wmin[w]);
+      if (a.dtBlock) store_block_dt(a.dtBlock, b, m);
+      atomicMin(&a.ts->DtMinBits, dbits(m));
     }
-    if (err) atomicOr(&a.ts->errFlag, kErrHlld);
-    __syncthreads();
-
-    double dtmin = 1e300;
-    if (t < NC) {
-      double o[8];
-#pragma unroll
-      for (int v = 0; v < 8; v++) o[v] = a.old[(size_t)b * 8 * NC + v * NC + t];
-      const int i = t % NI, j = t / NI;
-      double chg[8], divB = 0.0, vsum = 0.0, ub[6];
-#pragma unroll
-      for (int D = 0; D < S::NDIM; D++) {
-        const int f0 = D == 0 ? t : S::F0 + t, f1 = D == 0 ? (i + 1 < NI ? t + 1 : NC + j) : f0 + NI;
-#pragma unroll
-        for (int v = 0; v < 8; v++) {
-          const double d = fb[v * NF + f0] - fb[v * NF + f1];
-          chg[v] = D == 0 ? d : chg[v] + d;
-        }
-        const double e = mul_rn(g.invHalf[D], fb[9 * NF + f1] - fb[9 * NF + f0]);
-        divB = D == 0 ? e : divB + e;
-        const double x = fmax(fb[8 * NF + f0], fb[8 * NF + f1]);
-        vsum = D == 0 ? x : vsum + x;
-      }
-#pragma unroll
-      for (int q = 0; q < 6; q++) ub[q] = P[t + (kUx + q) * PT];
-      if (a.computeDt) dtmin = g.volume / vsum;
-      double *out = reinterpret_cast<double *>(a.out) + (size_t)b * 8 * NC + t;
-      update_cell<double>(a, DtNoCfl, g.invVolume, chg, divB, ub, o, out, NC);
-    }
-    if (a.computeDt) {
-      for (int off = 16; off > 0; off >>= 1) dtmin = fmin(dtmin, __shfl_xor_sync(0xffffffffu, dtmin, off));
-      if ((t & 31) == 0) wmin[t >> 5] = dtmin;
-      __syncthreads();
-      if (t == 0) {
-        double m = wmin[0];
-        for (int w = 1; w < S::NTHR / 32; w++) m = fmin(m, wmin[w]);
-        if (a.dtBlock) store_block_dt(a.dtBlock, b, m);
-        atomicMin(&a.ts->DtMinBits, (unsigned long long)__double_as_longlong(m));
-      }
-    }
-    __syncthreads();  // P and the slots are read
   }
   finish_stage(a);
 }
-
 }  // namespace bx
