@@ -5,11 +5,16 @@
 // IEEE divisions and square roots, no contraction: compiled with
 // --fmad=false).  Runs with the minmod limiter amplify the rounding of a step
 // in 2D: the flux functions of the 3D kernel, with a thread per face and 20
-// warps per SM, took 39 us per step at 384 x 384 where the kernel before took 87,
+// warps per SM, took 39 us per step at 384 x 384 where this kernel takes 78,
 // but gave digits up to 2e-14 of the norm apart after 50 steps.  Kept of that
-// are five CTAs per SM (128 registers instead of 255) and the end of the time
-// step in the last CTA.  The gather loads through the read-only path, so the
-// kernel does not start before the one that writes the state has ended.
+// is the end of the time step in the last CTA.  The gather loads through the
+// read-only path, so the kernel does not start before the one that writes the
+// state has ended.
+//
+// No limit on the registers: 128 (Rusanov), 148 (Linde), 122 (HLLD) and 212 (Roe)
+// hold five, four, five and three CTAs per SM without spills; a limit of 128
+// for five CTAs spilled 120 bytes of Linde's and 320 of Roe's: Linde 81.2 us
+// per step at 384 x 384 instead of 78.3, 23.0 instead of 21.2 on 10 x 9 blocks.
 #pragma once
 #include "bx_stage.cuh"
 
@@ -87,7 +92,7 @@ __device__ __forceinline__ void sweep(const StageArgs &a, const BlockGeom &g, co
 }
 
 template <class S, typename Real, typename InT, typename OutT, int FLUX>
-__global__ void __launch_bounds__(S::NTHREAD, 5) stage_flat_kernel(const StageArgs a) {
+__global__ void __launch_bounds__(S::NTHREAD) stage_flat_kernel(const StageArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Real *tile = reinterpret_cast<Real *>(smem_raw);
   Real *fbuf = tile + 8 * S::NT;
