@@ -17,15 +17,17 @@
 //               the 2x2 finer faces (tvd_reschange states, or the first-order
 //               states of get_faceX_first), their Vdt and their normal fields
 //               times FaceRatio = 1/4 (src/ModConserveFlux.f90:79-265),
-//               computed with the stage kernel's own primitive conversion and
-//               face_slots so that the coarse side and the finer blocks see
-//               the same fluxes
+//               computed with the primitive conversion and the flux code of
+//               the stage kernel that the grid runs (UNITS: rcp_cell and
+//               unit_flux of bx_stage_unit.cuh, else cell_rcp and face_slots
+//               of bx_stage3d.cuh) so that the coarse side and the finer
+//               blocks see the same fluxes
 //
 // The stage kernel copies the ghost slabs into its tile and, on the coarse
 // side, replaces its face slots by the sums (apply_cons_flux,
 // src/ModConserveFlux.f90:268-445).
 #include "bx_amr.h"
-#include "bx_stage3d.cuh"
+#include "bx_stage_unit.cuh"
 
 namespace bx {
 
@@ -131,13 +133,13 @@ __global__ void k_rc_ghost(const InT *__restrict__ in, const RcSlab *__restrict_
 }
 
 // primitive state of block-local cell c as the stage kernel's tile holds it
-template <int N, typename TileT, typename Real, typename InT>
+template <int N, typename TileT, typename Real, bool UNITS, typename InT>
 __device__ __forceinline__ void rc_prim(const InT *in, int blk, int c, Real (&P)[8]) {
   constexpr int NC = N * N * N;
   TileT p[8];
 #pragma unroll
   for (int v = 0; v < 8; v++) p[v] = (TileT)in[((size_t)blk * 8 + v) * NC + c];
-  const TileT rhoInv = TileT(1) / p[kRho];
+  const TileT rhoInv = UNITS ? rcp_cell(p[kRho]) : cell_rcp(p[kRho]);
   p[kUx] = rhoInv * p[kUx];
   p[kUy] = rhoInv * p[kUy];
   p[kUz] = rhoInv * p[kUz];
@@ -145,7 +147,7 @@ __device__ __forceinline__ void rc_prim(const InT *in, int blk, int c, Real (&P)
   for (int v = 0; v < 8; v++) P[v] = (Real)p[v];
 }
 
-template <int N, typename TileT, typename Real, int FLUX, int D>
+template <int N, typename TileT, typename Real, int FLUX, int D, bool UNITS>
 __device__ __forceinline__ void rc_face_sum(const StageArgs &a, const RcSlab &S, int t0, int t1, double *out) {
   const TileT *in = reinterpret_cast<const TileT *>(a.in);
   const int hi = S.side & 1;
@@ -163,13 +165,13 @@ __device__ __forceinline__ void rc_face_sum(const StageArgs &a, const RcSlab &S,
   // layer) and, for the TVD faces, the coarse cell beyond it and the finer
   // block's 2x2 cells next to the face and behind them
   Real Pc[8], Pc2[8], F1[4][8], F2[4][8];
-  rc_prim<N, TileT, Real>(in, S.block, cell(hi ? N - 1 : 0, t0, t1), Pc);
+  rc_prim<N, TileT, Real, UNITS>(in, S.block, cell(hi ? N - 1 : 0, t0, t1), Pc);
   const bool tvd = a.tvdRc != 0;
-  if (tvd) rc_prim<N, TileT, Real>(in, S.block, cell(hi ? N - 2 : 1, t0, t1), Pc2);
+  if (tvd) rc_prim<N, TileT, Real, UNITS>(in, S.block, cell(hi ? N - 2 : 1, t0, t1), Pc2);
 #pragma unroll
   for (int u = 0; u < 4; u++) {
-    rc_prim<N, TileT, Real>(in, F, cell(hi ? 0 : N - 1, a0 + (u & 1), a1 + (u >> 1)), F1[u]);
-    if (tvd) rc_prim<N, TileT, Real>(in, F, cell(hi ? 1 : N - 2, a0 + (u & 1), a1 + (u >> 1)), F2[u]);
+    rc_prim<N, TileT, Real, UNITS>(in, F, cell(hi ? 0 : N - 1, a0 + (u & 1), a1 + (u >> 1)), F1[u]);
+    if (tvd) rc_prim<N, TileT, Real, UNITS>(in, F, cell(hi ? 1 : N - 2, a0 + (u & 1), a1 + (u >> 1)), F2[u]);
   }
   const Real beta = (Real)fmin(a.betaRc, a.beta);
   const Real area = (Real)a.geom[F].area[D];
@@ -191,12 +193,25 @@ __device__ __forceinline__ void rc_face_sum(const StageArgs &a, const RcSlab &S,
       L[v] = hi ? c : f;
       R[v] = hi ? f : c;
     }
-    ok = face_slots<D, FLUX, Real>(L, R, (Real)a.gamma, (Real)a.invGm1, area, o, 1,
-                                   hi ? Pc[kBx + D] : F1[u][kBx + D], hi ? F1[u][kBx + D] : Pc[kBx + D],
-                                   hi ? Pc[kUx + D] : F1[u][kUx + D], hi ? F1[u][kUx + D] : Pc[kUx + D]) &&
-         ok;
+    const Real cbL = hi ? Pc[kBx + D] : F1[u][kBx + D], cbR = hi ? F1[u][kBx + D] : Pc[kBx + D];
+    const Real cuL = hi ? Pc[kUx + D] : F1[u][kUx + D], cuR = hi ? F1[u][kUx + D] : Pc[kUx + D];
+    if constexpr (UNITS) {
+      constexpr int T1 = (D + 1) % 3, T2 = (D + 2) % 3;
+      constexpr int var[8] = {0, 1 + D, 1 + T1, 1 + T2, 4 + D, 4 + T1, 4 + T2, 7};
+      Real l[8], r[8], bn;
+      bool okU = true;
 #pragma unroll
-    for (int m = 0; m < 9; m++) sum[m] = sum[m] + (double)o[m];
+      for (int q = 0; q < 8; q++) { l[q] = L[var[q]]; r[q] = R[var[q]]; }
+      o[8] = unit_flux<FLUX, Real>(D, l, r, (Real)a.gamma, (Real)a.invGm1, area, cbL, cbR, cuL, cuR, bn, okU,
+                                   [&](int q, Real f) { o[var[q]] = f; });
+      L[kBx + D] = l[4];  // as the Roe flux leaves them
+      R[kBx + D] = r[4];
+      ok = okU && ok;
+    } else {
+      ok = face_slots<D, FLUX, Real>(L, R, (Real)a.gamma, (Real)a.invGm1, area, o, 1, cbL, cbR, cuL, cuR) && ok;
+    }
+#pragma unroll
+    for (int m = 0; m < 9; m++) sum[m] = __dadd_rn(sum[m], (double)o[m]);  // the rounded flux, not contracted
     bnL = bnL + (double)L[kBx + D] * 0.25;
     bnR = bnR + (double)R[kBx + D] * 0.25;
   }
@@ -206,7 +221,7 @@ __device__ __forceinline__ void rc_face_sum(const StageArgs &a, const RcSlab &S,
   if (!ok) atomicOr(&a.ts->errFlag, kErrHlld);
 }
 
-template <int N, typename TileT, typename Real, int FLUX>
+template <int N, typename TileT, typename Real, int FLUX, bool UNITS>
 __global__ void k_rc_flux(const StageArgs a, const RcSlab *__restrict__ slabs, double *flux) {
   const RcSlab S = slabs[blockIdx.x];
   if (S.type != -1) return;
@@ -215,41 +230,58 @@ __global__ void k_rc_flux(const StageArgs a, const RcSlab *__restrict__ slabs, d
   const int t0 = f % N, t1 = f / N;
   double *out = flux + ((size_t)blockIdx.x * N * N + f) * kRcSlots;
   switch (S.side >> 1) {
-    case 0: rc_face_sum<N, TileT, Real, FLUX, 0>(a, S, t0, t1, out); break;
-    case 1: rc_face_sum<N, TileT, Real, FLUX, 1>(a, S, t0, t1, out); break;
-    default: rc_face_sum<N, TileT, Real, FLUX, 2>(a, S, t0, t1, out); break;
+    case 0: rc_face_sum<N, TileT, Real, FLUX, 0, UNITS>(a, S, t0, t1, out); break;
+    case 1: rc_face_sum<N, TileT, Real, FLUX, 1, UNITS>(a, S, t0, t1, out); break;
+    default: rc_face_sum<N, TileT, Real, FLUX, 2, UNITS>(a, S, t0, t1, out); break;
+  }
+}
+
+// 4^3 blocks always run in units, 8^3 blocks with the Roe flux never
+template <int N, typename TileT, typename Real, int FLUX>
+static void rc_flux_launch(bool units, const StageArgs &a, const RcSlab *slabs, int nSlab, double *fluxBuf,
+                           cudaStream_t st) {
+  if constexpr (N == 4) {
+    k_rc_flux<N, TileT, Real, FLUX, true><<<nSlab, N * N, 0, st>>>(a, slabs, fluxBuf);
+  } else {
+    if constexpr (FLUX != kFluxRoe) {
+      if (units) {
+        k_rc_flux<N, TileT, Real, FLUX, true><<<nSlab, N * N, 0, st>>>(a, slabs, fluxBuf);
+        return;
+      }
+    }
+    k_rc_flux<N, TileT, Real, FLUX, false><<<nSlab, N * N, 0, st>>>(a, slabs, fluxBuf);
   }
 }
 
 template <int N, typename TileT, typename Real>
-static cudaError_t rc_launch(int flux, const StageArgs &a, const RcSlab *slabs, int nSlab, const int *lc, int3 nRoot,
-                             double *ghost, double *fluxBuf, cudaStream_t st) {
+static cudaError_t rc_launch(int flux, bool units, const StageArgs &a, const RcSlab *slabs, int nSlab, const int *lc,
+                             int3 nRoot, double *ghost, double *fluxBuf, cudaStream_t st) {
   k_rc_ghost<N, TileT><<<nSlab, 2 * N * N, 0, st>>>(reinterpret_cast<const TileT *>(a.in), slabs, lc, nRoot, ghost,
                                                     a.tvdRc);
   switch (flux) {
-    case kFluxRusanov: k_rc_flux<N, TileT, Real, kFluxRusanov><<<nSlab, N * N, 0, st>>>(a, slabs, fluxBuf); break;
-    case kFluxLinde: k_rc_flux<N, TileT, Real, kFluxLinde><<<nSlab, N * N, 0, st>>>(a, slabs, fluxBuf); break;
-    case kFluxRoe: k_rc_flux<N, TileT, Real, kFluxRoe><<<nSlab, N * N, 0, st>>>(a, slabs, fluxBuf); break;
-    default: k_rc_flux<N, TileT, Real, kFluxHlld><<<nSlab, N * N, 0, st>>>(a, slabs, fluxBuf); break;
+    case kFluxRusanov: rc_flux_launch<N, TileT, Real, kFluxRusanov>(units, a, slabs, nSlab, fluxBuf, st); break;
+    case kFluxLinde: rc_flux_launch<N, TileT, Real, kFluxLinde>(units, a, slabs, nSlab, fluxBuf, st); break;
+    case kFluxRoe: rc_flux_launch<N, TileT, Real, kFluxRoe>(units, a, slabs, nSlab, fluxBuf, st); break;
+    default: rc_flux_launch<N, TileT, Real, kFluxHlld>(units, a, slabs, nSlab, fluxBuf, st); break;
   }
   return cudaGetLastError();
 }
 
-cudaError_t launch_reschange(int shape, int flux, int kind, const StageArgs &a, const RcSlab *slabs, int nSlab,
-                             const int *lc, int3 nRoot, double *ghost, double *fluxBuf, cudaStream_t st) {
+cudaError_t launch_reschange(int shape, int flux, int kind, bool units, const StageArgs &a, const RcSlab *slabs,
+                             int nSlab, const int *lc, int3 nRoot, double *ghost, double *fluxBuf, cudaStream_t st) {
   if (nSlab == 0) return cudaSuccess;
   const bool n8 = shape == kShape888;
   if (shape != kShape888 && shape != kShape444) return cudaErrorInvalidValue;
   switch (kind) {
     case kKindFp64:
-      return n8 ? rc_launch<8, double, double>(flux, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st)
-                : rc_launch<4, double, double>(flux, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st);
+      return n8 ? rc_launch<8, double, double>(flux, units, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st)
+                : rc_launch<4, double, double>(flux, units, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st);
     case kKindFp32In64:
-      return n8 ? rc_launch<8, double, float>(flux, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st)
-                : rc_launch<4, double, float>(flux, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st);
+      return n8 ? rc_launch<8, double, float>(flux, units, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st)
+                : rc_launch<4, double, float>(flux, units, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st);
     case kKindFp32In32:
-      return n8 ? rc_launch<8, float, float>(flux, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st)
-                : rc_launch<4, float, float>(flux, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st);
+      return n8 ? rc_launch<8, float, float>(flux, units, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st)
+                : rc_launch<4, float, float>(flux, units, a, slabs, nSlab, lc, nRoot, ghost, fluxBuf, st);
   }
   return cudaErrorInvalidValue;
 }

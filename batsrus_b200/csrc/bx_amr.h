@@ -53,8 +53,9 @@ cudaError_t launch_amr_remap(int shape, const double *in, double *out, const int
                              cudaStream_t st);
 
 // ghost slabs of all resolution-change sides and, for the coarse sides, the
-// summed finer fluxes; lc = level, ix, iy, iz per block
-cudaError_t launch_reschange(int shape, int flux, int kind, const StageArgs &a, const RcSlab *slabs, int nSlab,
-                             const int *lc, int3 nRoot, double *ghost, double *fluxBuf, cudaStream_t st);
+// summed finer fluxes; units: the stage runs in units (stage3d_units); lc =
+// level, ix, iy, iz per block
+cudaError_t launch_reschange(int shape, int flux, int kind, bool units, const StageArgs &a, const RcSlab *slabs,
+                             int nSlab, const int *lc, int3 nRoot, double *ghost, double *fluxBuf, cudaStream_t st);
 
 }  // namespace bx

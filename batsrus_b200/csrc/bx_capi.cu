@@ -352,6 +352,9 @@ StageArgs stage_args(int iStage, bool computeDt) {
   return a;
 }
 
+// whether the explicit stages of this 3D grid run in units
+bool in_units() { return stage3d_units(g.shape, g.sch.TypeFlux); }
+
 // one stage of all blocks (update_state_fast); the cell time steps are
 // computed in the last stage, or where computeDt asks for them.  finish:
 // StageArgs::finish, with the time limit tLimit
@@ -384,7 +387,7 @@ int launch_stage_dt(int iStage, bool computeDt, int finish = 0, double tLimit = 
       m = &g.mapY32;
     }
     if (g.nSlab) {
-      e = launch_reschange(g.shape, g.sch.TypeFlux, kind, a, g.slabs, g.nSlab, g.lcDev,
+      e = launch_reschange(g.shape, g.sch.TypeFlux, kind, in_units(), a, g.slabs, g.nSlab, g.lcDev,
                            make_int3(g.nRoot[0], g.nRoot[1], g.nRoot[2]), g.rcGhost, g.rcFlux, g.st);
       if (e != cudaSuccess) return fail(BX_ERR_CUDA, "resolution-change kernels: %s", cudaGetErrorString(e));
     }
@@ -452,7 +455,7 @@ int tune_stage_impl() {
             m = &g.mapY32;
           }
           if (g.nSlab)
-            e = launch_reschange(g.shape, g.sch.TypeFlux, kind, a, g.slabs, g.nSlab, g.lcDev,
+            e = launch_reschange(g.shape, g.sch.TypeFlux, kind, in_units(), a, g.slabs, g.nSlab, g.lcDev,
                                  make_int3(g.nRoot[0], g.nRoot[1], g.nRoot[2]), g.rcGhost, g.rcFlux, g.st);
           if (e == cudaSuccess) e = launch_stage3d(g.shape, g.sch.TypeFlux, kind, *m, a, g.nSM, g.st);
         }
@@ -495,7 +498,7 @@ int tune_stage_impl() {
 // (StageArgs::finish), a step is its stages: begin_steps sets the first
 // one's time step, every step but the last sets the next one's.  Elsewhere
 // each step is launched with its own set_dt and end_step kernels.
-bool fused_steps() { return !g.use3d || stage3d_finishes(g.shape, g.sch.TypeFlux); }
+bool fused_steps() { return !g.use3d || in_units(); }
 
 int begin_steps(double tLimit) {
   if (!fused_steps()) return BX_OK;

@@ -220,8 +220,9 @@ struct alignas(64) TmaMaps {
 enum { kKindFp64 = 0, kKindFp32In64 = 1, kKindFp32In32 = 2 };
 cudaError_t launch_stage3d(int shape, int flux, int kind, const TmaMaps &maps, const StageArgs &a, int nSM,
                            cudaStream_t st);
-// whether that kernel carries out StageArgs::finish
-bool stage3d_finishes(int shape, int flux);
+// whether an explicit stage runs in units (bx_stage_unit.cuh), which carry out
+// StageArgs::finish
+bool stage3d_units(int shape, int flux);
 enum { kPhaseFaceValue = 0, kPhaseFaceFlux = 1, kPhaseSource = 2, kPhaseUpdate = 3, kPhaseTimestep = 4 };
 
 }  // namespace bx

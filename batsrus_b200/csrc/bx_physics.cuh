@@ -598,7 +598,7 @@ __device__ __forceinline__ double fast_speed(double gp, double b2, double bn4, d
 }
 __device__ __forceinline__ float fast_speed(float gp, float b2, float bn4, float rho2) {
   const float i = 2.0f * frcp(rho2), s = gp * i, f = (gp + b2) * i;
-  return fsqrt(0.5f * (f + fsqrt(fmaxf(0.0f, f * f - s * (bn4 * i)))));
+  return fsqrt(0.5f * (f + fsqrt(fmaxf(0.0f, fmaf(f, f, -(s * (bn4 * i)))))));
 }
 
 // The 8 fluxes times area go to out(q, flux), q in the frame's order with the
@@ -660,37 +660,46 @@ __device__ __forceinline__ R flux_frame(const R (&L)[8], const R (&Rt)[8], R gam
   return vdt;
 }
 
+__device__ __forceinline__ float dot3(float a, float b, float c, float x, float y, float z) {
+  return fmaf(c, z, fmaf(b, y, a * x));
+}
+__device__ __forceinline__ double dot3(double a, double b, double c, double x, double y, double z) {
+  return fma(c, z, fma(b, y, a * x));
+}
+
 // hlld_flux with Linde's fix (get_numerical_flux, src/ModFaceFlux.f90:2130-2473,
 // 2826-3160) in the face's frame.  The formulas of the two sides of the
 // contact are mirror images, so the side that the contact moves away from
 // (near, sg = 1 for the left one) and the other (far) are selected once and
 // one copy of the code serves both: no divergence between faces with
-// opposite Un, half the instructions in the cache.  False where the
+// opposite Un, half the instructions in the cache.  The multiply-adds are
+// spelled out, so that every kernel rounds alike: the flux sums at a resolution
+// change (bx_amr.cu) must be those of the finer blocks.  False where the
 // reference stops (negative density ratio).
 template <typename R, class Out>
 __device__ __forceinline__ bool hlld_frame(const R (&L)[8], const R (&Rt)[8], R gamma, R invGm1, R area, R &vdt,
                                            const Out &out) {
   const R cTiny = R(1.0e-6);
   const R dBn = R(0.5) * (Rt[4] - L[4]), Bn = L[4] + dBn, Bn2 = Bn * Bn;
-  const R b2L = L[5] * L[5] + L[6] * L[6], b2R = Rt[5] * Rt[5] + Rt[6] * Rt[6];
+  const R b2L = fma(L[6], L[6], L[5] * L[5]), b2R = fma(Rt[6], Rt[6], Rt[5] * Rt[5]);
   const R cL = fast_speed(gamma * L[7], Bn2 + b2L, R(4) * Bn2, R(2) * L[0]);
   const R cR = fast_speed(gamma * Rt[7], Bn2 + b2R, R(4) * Bn2, R(2) * Rt[0]);
   const R sL = lo2(L[1] - cL, Rt[1] - cR), sR = hi2(L[1] + cL, Rt[1] + cR);
   const R cmax = hi2(sR, -sL);
   vdt = cmax * area;
-  const R ptL = L[7] + R(0.5) * (Bn2 + b2L), ptR = Rt[7] + R(0.5) * (Bn2 + b2R);
+  const R ptL = fma(R(0.5), Bn2 + b2L, L[7]), ptR = fma(R(0.5), Bn2 + b2R, Rt[7]);
   const R DsL = sL - L[1], DsR = sR - Rt[1], DrL = DsL * L[0], DrR = DsR * Rt[0];
   const R inv = rcp_nb(DrR - DrL);
-  const R Un = (DrR * Rt[1] - DrL * L[1] - ptR + ptL) * inv;
-  const R pt12 = (DrR * ptL - DrL * ptR + DrR * DrL * (Rt[1] - L[1])) * inv;
+  const R Un = (fma(DrR, Rt[1], -(DrL * L[1])) - ptR + ptL) * inv;
+  const R pt12 = fma(DrR * DrL, Rt[1] - L[1], fma(DrR, ptL, -(DrL * ptR))) * inv;
   const bool super = sL >= R(0) || sR <= R(0);
   const bool left = super ? sL >= R(0) : Un >= R(0);
   // near and far states: rho, u_n, u_t1, u_t2, b_t1, b_t2, p
   const R rN = left ? L[0] : Rt[0], uN = left ? L[1] : Rt[1], v1N = left ? L[2] : Rt[2], v2N = left ? L[3] : Rt[3];
   const R b1N = left ? L[5] : Rt[5], b2N = left ? L[6] : Rt[6], pN = left ? L[7] : Rt[7];
   const R ptN = left ? ptL : ptR;
-  const R eN = invGm1 * pN + (ptN - pN) + R(0.5) * (rN * (uN * uN + v1N * v1N + v2N * v2N));
-  const R ubN = uN * Bn + v1N * b1N + v2N * b2N;
+  const R eN = fma(R(0.5) * rN, dot3(uN, v1N, v2N, uN, v1N, v2N), fma(invGm1, pN, ptN - pN));
+  const R ubN = dot3(uN, v1N, v2N, Bn, b1N, b2N);
   R rho, un, v1, v2, b1, b2, pt, e, ub;
   bool ok = true;
   if (super) {
@@ -702,12 +711,12 @@ __device__ __forceinline__ bool hlld_frame(const R (&L)[8], const R (&Rt)[8], R 
     pt = pt12;
     // one outer star state: density factor, tangential velocity and field
     auto star = [&](R Ds, R Dr, R gap, R u, R w1, R w2, R c1, R c2, R &o1, R &o2, R &p1, R &p2) {
-      const R den = Dr * gap - Bn2;
+      const R den = fma(Dr, gap, -Bn2);
       const bool plain = den < cTiny;
       const R t = rcp_nb(plain ? R(1) : den);
-      const R fu = plain ? R(0) : Bn * (Un - u) * t, fb = plain ? R(1) : (Dr * Ds - Bn2) * t;
-      o1 = w1 - fu * c1;
-      o2 = w2 - fu * c2;
+      const R fu = plain ? R(0) : Bn * (Un - u) * t, fb = plain ? R(1) : fma(Dr, Ds, -Bn2) * t;
+      o1 = fma(-fu, c1, w1);
+      o2 = fma(-fu, c2, w2);
       p1 = c1 * fb;
       p2 = c2 * fb;
     };
@@ -715,10 +724,10 @@ __device__ __forceinline__ bool hlld_frame(const R (&L)[8], const R (&Rt)[8], R 
     R v1s, v2s, b1s, b2s;
     star(DsN, DrN, gapN, uN, v1N, v2N, b1N, b2N, v1s, v2s, b1s, b2s);
     rho = DrN * ig;
-    const R ubs = Un * Bn + v1s * b1s + v2s * b2s;
-    e = (DsN * eN - ptN * uN + pt12 * Un + Bn * (ubN - ubs)) * ig;
+    const R ubs = dot3(Un, v1s, v2s, Bn, b1s, b2s);
+    e = fma(Bn, ubN - ubs, fma(pt12, Un, fma(DsN, eN, -(ptN * uN)))) * ig;
     const R sqN = sqrt_nb(rho), aBn = fabs(Bn);
-    if (sg * Un - div_nb(aBn, sqN) >= R(0)) {
+    if (fma(sg, Un, -div_nb(aBn, sqN)) >= R(0)) {
       v1 = v1s; v2 = v2s; b1 = b1s; b2 = b2s; ub = ubs;
     } else {
       // between the Alfven waves
@@ -731,23 +740,23 @@ __device__ __forceinline__ bool hlld_frame(const R (&L)[8], const R (&Rt)[8], R 
       R v1f, v2f, b1f, b2f;
       star(DsF, DrF, gapF, uF, v1F, v2F, b1F, b2F, v1f, v2f, b1f, b2f);
       const R t = rcp_nb(sqN + sqF), sB = copysign(R(1), Bn), ss = sg * sB, sNF = sqN * sqF * ss;
-      v1 = (sqN * v1s + sqF * v1f + (b1f - b1s) * ss) * t;
-      v2 = (sqN * v2s + sqF * v2f + (b2f - b2s) * ss) * t;
-      b1 = (sqN * b1f + sqF * b1s + (v1f - v1s) * sNF) * t;
-      b2 = (sqN * b2f + sqF * b2s + (v2f - v2s) * sNF) * t;
-      ub = Un * Bn + v1 * b1 + v2 * b2;
-      e = e - ss * (sqN * (ubs - ub));
+      v1 = fma(b1f - b1s, ss, fma(sqF, v1f, sqN * v1s)) * t;
+      v2 = fma(b2f - b2s, ss, fma(sqF, v2f, sqN * v2s)) * t;
+      b1 = fma(v1f - v1s, sNF, fma(sqF, b1s, sqN * b1f)) * t;
+      b2 = fma(v2f - v2s, sNF, fma(sqF, b2s, sqN * b2f)) * t;
+      ub = dot3(Un, v1, v2, Bn, b1, b2);
+      e = fma(-ss, sqN * (ubs - ub), e);
     }
   }
   const R m = area * (rho * un), aB = area * Bn, au = area * un;
   out(0, m);
-  out(1, m * un - aB * Bn + area * pt);
-  out(2, m * v1 - aB * b1);
-  out(3, m * v2 - aB * b2);
+  out(1, fma(m, un, fma(-aB, Bn, area * pt)));
+  out(2, fma(m, v1, -(aB * b1)));
+  out(3, fma(m, v2, -(aB * b2)));
   out(4, -(vdt * dBn));
-  out(5, au * b1 - aB * v1);
-  out(6, au * b2 - aB * v2);
-  out(7, au * (e + pt) - aB * ub - vdt * (Bn * dBn));
+  out(5, fma(au, b1, -(aB * v1)));
+  out(6, fma(au, b2, -(aB * v2)));
+  out(7, fma(au, e + pt, fma(-aB, ub, -(vdt * (Bn * dBn)))));
   return ok;
 }
 

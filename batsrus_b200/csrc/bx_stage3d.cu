@@ -9,7 +9,7 @@
 
 namespace bx {
 
-bool stage3d_finishes(int shape, int flux) {
+bool stage3d_units(int shape, int flux) {
   if (shape == kShape444) return true;
   return flux != kFluxRoe && (tune_value(kTuneStageVariant) == 0 || tune_value(kTuneStageVariant) == 3);
 }
