@@ -25,7 +25,10 @@ UNITS = [
     ("bx_stage_flat.cu", ["--fmad=false"]),
     ("bx_stage3d.cu", []),
     ("bx_stage3d_fpt2.cu", []),
-    ("bx_stage3d_v2.cu", []),
+    ("bx_stage8_rusanov.cu", []),
+    ("bx_stage8_linde.cu", []),
+    ("bx_stage8_hlld.cu", []),
+    ("bx_stage8_roe.cu", []),
     ("bx_stage_unit_rusanov.cu", []),
     ("bx_stage_unit_linde.cu", []),
     ("bx_stage_unit_hlld.cu", []),
@@ -39,7 +42,7 @@ UNITS = [
     ("bx_tune.cu", []),
     ("bx_capi.cu", []),
 ]
-HEADERS = ["bx_physics.cuh", "bx_stage.cuh", "bx_device.h", "bx_stage3d.cuh", "bx_stage3d_v2.cuh", "bx_stage3d_launch.cuh", "bx_stage_unit.cuh", "bx_stage_flat.cuh", "bx_stage_line.cuh",
+HEADERS = ["bx_physics.cuh", "bx_stage.cuh", "bx_device.h", "bx_stage3d.cuh", "bx_stage3d_v2.cuh", "bx_stage3d_launch.cuh", "bx_stage8_launch.cuh", "bx_stage_unit.cuh", "bx_stage_flat.cuh", "bx_stage_line.cuh",
            "bx_stage_unit_launch.cuh", "bx_tma.cuh", "bx_core.h",
            "bx_impl_kernels.cuh", "bx_krylov.cuh", "bx_tune.h", "bx_tc.cuh", "bx_learned.cuh", "bx_learned_kernels.cuh", "bx_amr.h"]
 

@@ -5,33 +5,39 @@
 // and writes FP64; the reconstruction and fluxes run in FP32, the
 // conserved-state update and the pressure recovery in FP64.
 #include "bx_stage3d_launch.cuh"
+#include "bx_stage8_launch.cuh"
 #include "bx_stage_unit_launch.cuh"
 
 namespace bx {
 
 bool stage3d_units(int shape, int flux) {
-  if (shape == kShape444) return true;
-  return flux != kFluxRoe && (tune_value(kTuneStageVariant) == 0 || tune_value(kTuneStageVariant) == 3);
+  return shape == kShape444 || (flux != kFluxRoe && tune_value(kTuneStageVariant) == 0);
 }
+
+namespace {
+
+template <int FLUX>
+cudaError_t launch_blocks(int shape, int kind, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
+  // the implicit residual, whose finite-difference products amplify
+  // rounding, keeps the reference's order of operations (flux_lean)
+  if (shape == kShape888 && (a.outputResidual || !stage3d_units(shape, FLUX)))
+    return launch_stage8<FLUX>(kind, maps, a, nSM, st);
+  if (a.outputResidual) return launch_one<4, 1, double, double, double, FLUX>(maps, a, nSM, st);
+  return launch_unit<FLUX>(shape, kind, maps, a, nSM, st);
+}
+
+}  // namespace
 
 cudaError_t launch_stage3d(int shape, int flux, int kind, const TmaMaps &maps, const StageArgs &a, int nSM,
                            cudaStream_t st) {
   const int variant = shape == kShape888 ? tune_value(kTuneStageVariant) : 0;
   if (variant == 1) return launch_kind<8, 1>(flux, kind, maps, a, nSM, st);
   if (variant == 2) return launch_stage3d_fpt2(flux, kind, maps, a, nSM, st);
-  if (a.outputResidual) {
-    // the implicit residual, whose finite-difference products amplify
-    // rounding, keeps the reference's order of operations (flux_lean)
-    if (shape == kShape888) return launch_stage8_residual(flux, maps, a, nSM, st);
-    return launch_flux<4, 1, double, double, double>(flux, maps, a, nSM, st);
-  }
   switch (flux) {
-    case kFluxRusanov: return launch_unit<kFluxRusanov>(shape, kind, maps, a, nSM, st);
-    case kFluxLinde: return launch_unit<kFluxLinde>(shape, kind, maps, a, nSM, st);
-    case kFluxHlld: return launch_unit<kFluxHlld>(shape, kind, maps, a, nSM, st);
-    case kFluxRoe:
-      if (shape == kShape888) return launch_stage8_roe(kind, maps, a, nSM, st);
-      return launch_unit<kFluxRoe>(shape, kind, maps, a, nSM, st);
+    case kFluxRusanov: return launch_blocks<kFluxRusanov>(shape, kind, maps, a, nSM, st);
+    case kFluxLinde: return launch_blocks<kFluxLinde>(shape, kind, maps, a, nSM, st);
+    case kFluxHlld: return launch_blocks<kFluxHlld>(shape, kind, maps, a, nSM, st);
+    case kFluxRoe: return launch_blocks<kFluxRoe>(shape, kind, maps, a, nSM, st);
   }
   return cudaErrorInvalidValue;
 }

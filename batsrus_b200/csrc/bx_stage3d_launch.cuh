@@ -68,9 +68,5 @@ static cudaError_t launch_kind(int flux, int kind, const TmaMaps &maps, const St
 // 8^3 blocks with two faces per thread (bx_stage3d_fpt2.cu)
 cudaError_t launch_stage3d_fpt2(int flux, int kind, const TmaMaps &maps, const StageArgs &a, int nSM,
                                 cudaStream_t st);
-// 8^3 blocks: the implicit residual, and the explicit stages with the Roe
-// flux (bx_stage3d_v2.cu)
-cudaError_t launch_stage8_residual(int flux, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st);
-cudaError_t launch_stage8_roe(int kind, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st);
 
 }  // namespace bx

@@ -1,0 +1,7 @@
+// bx_stage8_rusanov.cu -- the stage kernel of whole 8^3 blocks with the Rusanov flux.
+#define BX_STAGE8_INSTANTIATE
+#include "bx_stage8_launch.cuh"
+
+namespace bx {
+template cudaError_t launch_stage8<kFluxRusanov>(int, const TmaMaps &, const StageArgs &, int, cudaStream_t);
+}

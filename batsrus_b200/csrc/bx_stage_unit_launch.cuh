@@ -68,7 +68,7 @@ cudaError_t launch_unit(int shape, int kind, const TmaMaps &maps, const StageArg
   // CTAs per SM: 3 of 128 registers in FP64, 4 of 96 in FP32 (160^3 Linde:
   // FP64 1286 us per step, 1460 with 2; FP32-bulk 748, 815 with 3 and 812 with 5)
   if (shape == kShape444) return launch_unit_kind<4, 3, 4, FLUX>(kind, maps, a, nSM, st);
-  if constexpr (FLUX == kFluxRoe) return cudaErrorInvalidValue;  // launch_stage8_roe
+  if constexpr (FLUX == kFluxRoe) return cudaErrorInvalidValue;  // launch_stage8
   else return launch_unit_kind<8, 3, 4, FLUX>(kind, maps, a, nSM, st);
 }
 #endif  // BX_UNIT_INSTANTIATE
