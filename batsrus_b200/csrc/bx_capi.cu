@@ -61,6 +61,7 @@ struct Ctx {
   double *scrL[3] = {}, *scrR[3] = {}, *scrF[3] = {}, *scrSrc = nullptr, *scrDt = nullptr;
   std::vector<char> touched;
   int *touchedDev = nullptr;  // device list of the blocks updated per block
+  int nRcBlock = 0;           // of them, blocks with a side at a resolution change
   int nOwned = 0;             // blocks 0..nOwned-1 are updated (one rank of a partitioned grid)
   int *haloIdx = nullptr;     // device list of blocks for bx_halo_pack / bx_halo_unpack
   bool compatPending = false;
@@ -329,6 +330,8 @@ void set_reschange(StageArgs &a) {
   bool anyFloat = false;
   for (int q = 0; q < 6; q++) anyFloat = anyFloat || g.typeBc[q] == BX_BC_FLOAT;
   a.anySpecial = g.nSlab > 0 || (sharp && anyFloat);
+  a.nRcBlock = g.nRcBlock;
+  a.isRank = g.nOwned < g.nBlock;
 }
 
 StageArgs stage_args(int iStage, bool computeDt) {
@@ -353,7 +356,10 @@ StageArgs stage_args(int iStage, bool computeDt) {
 }
 
 // whether the explicit stages of this 3D grid run in units
-bool in_units() { return stage3d_units(g.shape, g.sch.TypeFlux); }
+bool in_units() {
+  const int kind = g.sch.Precision == BX_FP64 ? kKindFp64 : kKindFp32In32;
+  return stage3d_units(g.shape, g.sch.TypeFlux, kind, stage_args(1, false), g.nSM);
+}
 
 // one stage of all blocks (update_state_fast); the cell time steps are
 // computed in the last stage, or where computeDt asks for them.  finish:
@@ -746,6 +752,11 @@ int bx_init(const bx_grid_desc *gd, const bx_scheme_params *sp) {
     }
   }
   g.nSlab = (int)g.slabsH.size();
+  g.nRcBlock = 0;
+  for (int b = 0; b < g.nOwned; b++) {
+    const int *t = &g.rcTypeH[6 * (size_t)b];
+    g.nRcBlock += std::any_of(t, t + 6, [](int v) { return v != 0; });
+  }
   if (g.nSlab && g.shape != kShape888 && g.shape != kShape444)
     return fail(BX_ERR_ARG, "resolution changes need 3D 8x8x8 or 4x4x4 blocks");
   // Morton processing order (L2 reuse of the neighbours' interiors) of the

@@ -121,6 +121,8 @@ struct StageArgs {
   // resolution change, and no sharper limiter next to a float boundary):
   // the stage kernel is then launched without that code
   int anySpecial = 1;
+  int nRcBlock = 0;  // updated blocks with a side at a resolution change
+  int isRank = 0;    // the blocks are one rank's part of a grid
 };
 
 #ifdef __CUDACC__
@@ -222,7 +224,7 @@ cudaError_t launch_stage3d(int shape, int flux, int kind, const TmaMaps &maps, c
                            cudaStream_t st);
 // whether an explicit stage runs in units (bx_stage_unit.cuh), which carry out
 // StageArgs::finish
-bool stage3d_units(int shape, int flux);
+bool stage3d_units(int shape, int flux, int kind, const StageArgs &a, int nSM);
 enum { kPhaseFaceValue = 0, kPhaseFaceFlux = 1, kPhaseSource = 2, kPhaseUpdate = 3, kPhaseTimestep = 4 };
 
 }  // namespace bx

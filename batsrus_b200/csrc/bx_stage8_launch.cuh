@@ -1,6 +1,7 @@
 // bx_stage8_launch.cuh -- launcher templates of the single-face-phase stage
-// kernel for 8^3 blocks (bx_stage3d_v2.cuh): the Roe flux, the residual of the
-// implicit step and stage_variant 3; one translation unit per flux instantiates them (bx_stage8_*.cu).  Roe's long
+// kernel for 8^3 blocks (bx_stage3d_v2.cuh): grids with resolution changes
+// (stage3d_units), the Roe flux, the residual of the implicit step and
+// stage_variant 3; one translation unit per flux instantiates them (bx_stage8_*.cu).  Roe's long
 // face code runs better here, with one set of barriers per block and 128
 // registers (96^3: 665 us per FP64 step and 368 per FP32-bulk step, against
 // 800 and 420 in units of 128 cells).
@@ -55,12 +56,14 @@ template <int FLUX>
 cudaError_t launch_stage8(int kind, const TmaMaps &maps, const StageArgs &a, int nSM, cudaStream_t st) {
   // FP64: one CTA per SM (the FP64 tile and face slots fill the shared
   // memory) of 512 threads, or 576 (three face groups per warp, 96 registers)
-  // with stage_variant 3.  FP32-bulk: one CTA of 512 per SM or, for
-  // stage_ctas_per_sm >= 2, two CTAs of 256, each on its own block
+  // with stage_variant 3 and on grids with resolution changes (us per step,
+  // 8^3 roots and three levels: HLLD 1498 against 2180, Linde 1249 against
+  // 1696).  FP32-bulk: one CTA of 512 per SM or, for stage_ctas_per_sm >= 2,
+  // two CTAs of 256, each on its own block
   const bool two = tune_value(kTuneStageGrid) >= 2;
   switch (kind) {
     case kKindFp64:
-      if (tune_value(kTuneStageVariant) == 3)
+      if (tune_value(kTuneStageVariant) == 3 || (FLUX != kFluxRoe && a.nRcBlock > 0))
         return launch8_flux<576, 1, double, double, double, FLUX>(maps, a, nSM, st);
       return launch8_flux<512, 1, double, double, double, FLUX>(maps, a, nSM, st);
     case kKindFp32In64:
