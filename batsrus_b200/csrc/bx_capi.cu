@@ -68,8 +68,8 @@ struct Ctx {
   int iStage = 1;
   cudaStream_t st = nullptr;
   cudaGraphExec_t graph = nullptr;
-  double graphTLimit = 0;
-  bool graphFused = false;
+  bool graphFused = false;     // its steps end in the stage kernel (fused_steps)
+  double graphTLimit = 0;      // its time limit, where they do not
   int graphSteps = 1;  // time steps captured in one CUDA graph
   // TMA tensor maps of the two state buffers (3D shapes)
   bool use3d = false;
@@ -182,6 +182,14 @@ __global__ void soa_to_aos(const double *__restrict__ soa, double *__restrict__ 
 }
 
 __global__ void set_dt_kernel(StepState *ts, double tLimit, int useDtFixed, double dtFixed, double cfl) {
+  step_set_dt(ts, tLimit, useDtFixed, dtFixed, cfl);
+}
+
+// the start of a bx_advance whose steps end in the stage kernel
+__global__ void begin_steps_kernel(StepState *ts, int nStep, double tLimit, int useDtFixed, double dtFixed,
+                                   double cfl) {
+  ts->nLeft = nStep;
+  ts->tLimit = tLimit;
   step_set_dt(ts, tLimit, useDtFixed, dtFixed, cfl);
 }
 
@@ -362,12 +370,10 @@ bool in_units() {
 }
 
 // one stage of all blocks (update_state_fast); the cell time steps are
-// computed in the last stage, or where computeDt asks for them.  finish:
-// StageArgs::finish, with the time limit tLimit
-int launch_stage_dt(int iStage, bool computeDt, int finish = 0, double tLimit = -1.0) {
+// computed in the last stage, or where computeDt asks for them
+int launch_stage_dt(int iStage, bool computeDt, bool finish = false) {
   StageArgs a = stage_args(iStage, computeDt);
   a.finish = finish;
-  a.tLimit = tLimit;
   a.useDtFixed = g.sch.UseDtFixed;
   a.dtFixed = g.sch.DtFixed;
   if (g.timing) {
@@ -502,26 +508,24 @@ int tune_stage_impl() {
 
 // The time steps of bx_advance.  Where the stage kernel ends the step itself
 // (StageArgs::finish), a step is its stages: begin_steps sets the first
-// one's time step, every step but the last sets the next one's.  Elsewhere
-// each step is launched with its own set_dt and end_step kernels.
+// one's time step, and each step sets the next one's while some are left.
+// Elsewhere each step is launched with its own set_dt and end_step kernels.
 bool fused_steps() { return !g.use3d || in_units(); }
 
-int begin_steps(double tLimit) {
-  if (!fused_steps()) return BX_OK;
-  set_dt_kernel<<<1, 1, 0, g.st>>>(g.ts, tLimit, g.sch.UseDtFixed, g.sch.DtFixed, g.sch.Cfl);
+int begin_steps(int nStep, double tLimit) {
+  begin_steps_kernel<<<1, 1, 0, g.st>>>(g.ts, nStep, tLimit, g.sch.UseDtFixed, g.sch.DtFixed, g.sch.Cfl);
   CK(cudaGetLastError());
   return BX_OK;
 }
 
-int launch_step(double tLimit, bool last) {
-  const bool fused = fused_steps();
+int launch_step(bool fused, double tLimit) {
   if (!fused) {
     set_dt_kernel<<<1, 1, 0, g.st>>>(g.ts, tLimit, g.sch.UseDtFixed, g.sch.DtFixed, g.sch.Cfl);
     CK(cudaGetLastError());
   }
   for (int s = 1; s <= g.sch.nStage; s++) {
     const bool end = s == g.sch.nStage;
-    int r = launch_stage_dt(s, end, fused && end ? (last ? 1 : 2) : 0, tLimit);
+    int r = launch_stage_dt(s, end, fused && end);
     if (r) return r;
   }
   if (!fused) {
@@ -1216,22 +1220,19 @@ int bx_advance(int nStep, double tLimit) {
   NEED_READY();
   if (nStep < 0) return fail(BX_ERR_ARG, "nStep=%d", nStep);
   if (nStep == 0) return check_err_flag();
-  int r = begin_steps(tLimit);
-  if (r) return r;
-  // a graph holds steps that are followed by another one; the last step of
-  // the call is launched directly
-  const bool useGraph = !g.timing && g.sch.nStage == 2;
-  int n = 0;
-  if (useGraph && nStep > 1 && (!g.graph || g.graphTLimit != tLimit || g.graphFused != fused_steps())) {
+  const bool useGraph = !g.timing && g.sch.nStage == 2, fused = fused_steps();
+  int r = BX_OK, n = 0;
+  if (fused && (r = begin_steps(nStep, tLimit))) return r;
+  if (useGraph && (!g.graph || g.graphFused != fused || (!fused && g.graphTLimit != tLimit))) {
     // the first step of a new graph runs uncaptured, so that kernel
     // attributes are set before capture begins
-    if ((r = launch_step(tLimit, false))) return r;
+    if ((r = launch_step(fused, tLimit))) return r;
     n++;
     if (g.graph) { cudaGraphExecDestroy(g.graph); g.graph = nullptr; }
     cudaGraph_t gr;
     CK(cudaStreamBeginCapture(g.st, cudaStreamCaptureModeThreadLocal));
     for (int q = 0; q < g.graphSteps && !r; q++) {
-      r = launch_step(tLimit, false);
+      r = launch_step(fused, tLimit);
       g.nLaunchTotal -= g.sch.nStage;  // captured, not launched
     }
     cudaError_t e = cudaStreamEndCapture(g.st, &gr);
@@ -1239,16 +1240,16 @@ int bx_advance(int nStep, double tLimit) {
     if (e != cudaSuccess) return fail(BX_ERR_CUDA, "graph capture: %s", cudaGetErrorString(e));
     CK(cudaGraphInstantiate(&g.graph, gr, 0));
     cudaGraphDestroy(gr);
+    g.graphFused = fused;
     g.graphTLimit = tLimit;
-    g.graphFused = fused_steps();
   }
   while (n < nStep) {
-    if (useGraph && g.graph && nStep - 1 - n >= g.graphSteps) {
+    if (useGraph && nStep - n >= g.graphSteps) {
       CK(cudaGraphLaunch(g.graph, g.st));
       g.nLaunchTotal += g.sch.nStage * g.graphSteps;
       n += g.graphSteps;
     } else {
-      if ((r = launch_step(tLimit, n == nStep - 1))) return r;
+      if ((r = launch_step(fused, tLimit))) return r;
       n++;
     }
   }

@@ -23,6 +23,8 @@ struct StepState {
   int nStep;
   int errFlag;
   unsigned nDone;                 // CTAs of the step's last stage that are through (finish_stage)
+  int nLeft;                      // steps of the running bx_advance that are not through, and
+  double tLimit;                  // its time limit (finish_stage)
 };
 
 // Floors of the updated state, each active where > 0: RhoMin_I (the
@@ -88,11 +90,11 @@ struct StageArgs {
   int iStage, nStage, nOrder, limiter, useDivb, useHalfStep, computeDt;
   double beta, gamma, invGm1, cfl;
   double dtFactor = 0.0;   // the stage's part of the time step: cfl, or cfl iStage/nStage (half step scheme)
-  // the step's last stage: 0 nothing more, 1 its last CTA ends the time step,
-  // 2 and sets the next one's time step (set_global_timestep)
+  // the step's last stage: its last CTA ends the time step and, while steps
+  // are left, sets the next one's time step (set_global_timestep)
   int finish = 0;
   int useDtFixed = 0;
-  double dtFixed = 0.0, tLimit = -1.0;
+  double dtFixed = 0.0;
   // residual mode of the 3D kernel (get_residual of the implicit scheme):
   // the input holds total energy in the pressure slot, the output is the
   // increment dtScale*DtMax_CB*(S + dF/V) of the implicit variables, with
@@ -156,7 +158,8 @@ cudaError_t launch_dependent(void (*k)(P...), int grid, int block, size_t smem, 
 // access to the time-step state: the last CTA through ends the time step and
 // sets the next one's, in place of two launches of one thread each (5 us of
 // a step's 23 on a grid of 16^3).  Every CTA has read DtNoCfl and added its
-// minimum before it counts itself.
+// minimum before it counts itself.  The steps left and the time limit are
+// read from the state, so that the launches of all steps are alike.
 __device__ __forceinline__ void finish_stage(const StageArgs &a) {
   if (!a.finish) return;
   __syncthreads();
@@ -170,14 +173,17 @@ __device__ __forceinline__ void finish_stage(const StageArgs &a) {
       s.tSimulation = a.ts->tSimulation;
       s.nStep = a.ts->nStep;
       s.DtMinBits = atomicAdd(&a.ts->DtMinBits, 0ull);
-      step_end(&s, a.nStage, a.tLimit);
-      if (a.finish == 2) step_set_dt(&s, a.tLimit, a.useDtFixed, a.dtFixed, a.cfl);
+      const double tLimit = a.ts->tLimit;
+      const int nLeft = a.ts->nLeft - 1;
+      step_end(&s, a.nStage, tLimit);
+      if (nLeft > 0) step_set_dt(&s, tLimit, a.useDtFixed, a.dtFixed, a.cfl);
       a.ts->DtNoCfl = s.DtNoCfl;
       a.ts->Dt = s.Dt;
       a.ts->tSimulation = s.tSimulation;
       a.ts->nStep = s.nStep;
       a.ts->DtMinBits = s.DtMinBits;
       a.ts->nDone = 0;
+      a.ts->nLeft = nLeft;
     }
   }
 }
