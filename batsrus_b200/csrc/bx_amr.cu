@@ -19,8 +19,8 @@
 //               times FaceRatio = 1/4 (src/ModConserveFlux.f90:79-265),
 //               computed with the primitive conversion and the flux code of
 //               the stage kernel that the grid runs (UNITS: rcp_cell and
-//               unit_flux of bx_stage_unit.cuh, else cell_rcp and face_slots
-//               of bx_stage3d.cuh) so that the coarse side and the finer
+//               unit_flux of bx_stage_unit.cuh, else 1/rho and face_slots of
+//               bx_stage3d.cuh) so that the coarse side and the finer
 //               blocks see the same fluxes
 //
 // The stage kernel copies the ghost slabs into its tile and, on the coarse
@@ -139,7 +139,7 @@ __device__ __forceinline__ void rc_prim(const InT *in, int blk, int c, Real (&P)
   TileT p[8];
 #pragma unroll
   for (int v = 0; v < 8; v++) p[v] = (TileT)in[((size_t)blk * 8 + v) * NC + c];
-  const TileT rhoInv = UNITS ? rcp_cell(p[kRho]) : cell_rcp(p[kRho]);
+  const TileT rhoInv = UNITS ? rcp_cell(p[kRho]) : TileT(1) / p[kRho];
   p[kUx] = rhoInv * p[kUx];
   p[kUy] = rhoInv * p[kUy];
   p[kUz] = rhoInv * p[kUz];

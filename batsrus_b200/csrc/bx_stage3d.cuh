@@ -151,14 +151,6 @@ __device__ __forceinline__ int face_id(int i, int j, int k) {
   return i + N * (j + N * k);
 }
 
-// 1/rho of the conversion: IEEE in double; in float one Newton step on the
-// hardware approximation (IEEE rounding but for rare last bits), branch-free
-__device__ __forceinline__ double cell_rcp(double x) { return 1.0 / x; }
-__device__ __forceinline__ float cell_rcp(float x) {
-  const float y = frcp(x);
-  return fmaf(fmaf(-x, y, 1.0f), y, y);
-}
-
 // the ten face slots of one face from its left and right primitive states:
 // fluxes times area (0..7), Vdt (8), BnL + BnR (9); false where hlld_flux
 // stops.  cbL, cbR, cuL, cuR: the normal field and normal velocity of the
@@ -466,7 +458,7 @@ __global__ void __launch_bounds__(T::NTHR, 1)
                           (pb - TileT(0.5) * (prim[m][kUx] * prim[m][kUx] + prim[m][kUy] * prim[m][kUy] +
                                               prim[m][kUz] * prim[m][kUz]) / prim[m][kRho]);
           }
-          const TileT rhoInv = cell_rcp(prim[m][kRho]);
+          const TileT rhoInv = TileT(1) / prim[m][kRho];
           prim[m][kUx] = rhoInv * prim[m][kUx];
           prim[m][kUy] = rhoInv * prim[m][kUy];
           prim[m][kUz] = rhoInv * prim[m][kUz];

@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(B::NTHR, B::MINB)
         w[kP] = (TileT)(a.gamma - 1.0) *
                 (pb - TileT(0.5) * (w[kUx] * w[kUx] + w[kUy] * w[kUy] + w[kUz] * w[kUz]) / w[kRho]);
       }
-      const TileT rhoInv = cell_rcp(w[kRho]);
+      const TileT rhoInv = TileT(1) / w[kRho];
       w[kUx] = rhoInv * w[kUx];
       w[kUy] = rhoInv * w[kUy];
       w[kUz] = rhoInv * w[kUz];

@@ -198,9 +198,9 @@ __device__ __forceinline__ void cell_faces(int D, int i, int j, int k, int &f0, 
   }
 }
 
-// 1/rho of the conversion, branch-free in both precisions
+// 1/rho of the conversion: branch-free in double; in float the IEEE quotient
 __device__ __forceinline__ double rcp_cell(double x) { return rcp_nb(x); }
-__device__ __forceinline__ float rcp_cell(float x) { return cell_rcp(x); }
+__device__ __forceinline__ float rcp_cell(float x) { return 1.0f / x; }
 
 // a product that is not contracted into a sum: the three terms of div B
 // cancel, and one rounded product less leaves a spurious remainder
