@@ -48,10 +48,18 @@ __device__ __forceinline__ float fsqrt(float a) {
 // then one third-order step of the binomial series: with e = 1 - a y,
 // 1/a = y (1 + e + e^2 + ...); with e = 1 - a y^2,
 // 1/sqrt(a) = y (1 + e/2 + 3 e^2/8 + ...).  The neglected term is of the order of
-// e^3 = 2^-60, so the result is within one unit in the last place; the
-// quotient is corrected once with its remainder.  Normal operands; a zero
-// operand gives NaN where the IEEE operation gives infinity (sqrt_nb: the
-// callers add a tiny number that keeps the argument from zero).
+// e^3 = 2^-60.  Errors in units of the last place over 4 million operands:
+// rcp_nb 0.506 (0.2 % of the results are not the IEEE ones), div_nb, which
+// is corrected by its remainder, 0.5 (all are), sqrt_nb 0.76, over_sqrt_nb 1.43
+// (its bound: two roundings and half of a third, 2.5).  In the explicit 3D
+// kernel the IEEE operations in their place change nothing in the error of a run
+// against 64 bits (mean over 36 runs within 0.4 %, either way) and cost 43 %
+// (160^3 Linde, 1230 against 1765 us per step).
+// Operands: normal numbers whose result is normal.  A zero, infinite or
+// subnormal divisor gives NaN where the IEEE operation gives infinity, zero or a
+// number: a density or a wave-speed sum that is one of these is not a state
+// the scheme can advance.  Square roots of quantities that can be zero (a
+// pressure, a field) add a tiny number that keeps the argument from zero.
 __device__ __forceinline__ double rcp_nb(double a) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));

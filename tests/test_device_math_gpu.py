@@ -1,6 +1,13 @@
 """The reciprocals, quotients and square roots that the 3D stage kernels use,
 compiled from the kernels' own headers into a small library.  1/rho in float is
-the IEEE quotient: every mantissa, and zeros, infinities and subnormals."""
+the IEEE quotient: every mantissa, and zeros, infinities and subnormals.  The
+branch-free double forms are compared with extended precision.  Their errors
+in units of the last place (relative 2^-53 is half of one to one unit):
+  rcp_nb         the series' remainder e^3 (2^-60) and one rounding: 0.51
+  div_nb         the remainder of the quotient corrects it: 0.5
+  over_sqrt_nb   s = num y and the last sum round once each, the rounding of a y
+                 enters e and half of it the result: 2.5 at most (measured 1.43;
+                 with num = a 0.76)"""
 import ctypes
 import os
 import subprocess
@@ -92,3 +99,34 @@ def test_float_reciprocal_is_the_ieee_quotient(lib):
     with np.errstate(divide="ignore", over="ignore"):
         ref = np.float32(1.0) / x
     assert np.array_equal(o.view(np.uint32), ref.view(np.uint32)), int((o.view(np.uint32) != ref.view(np.uint32)).sum())
+
+
+@pytest.mark.parametrize("op,name,bound", [(0, "rcp_nb", 0.51), (1, "div_nb", 0.5), (2, "over_sqrt_nb", 2.5),
+                                           (3, "sqrt_nb", 2.5)])
+def test_double_forms_against_extended_precision(lib, op, name, bound):
+    """2^20 random operands and as many with mantissas next to 1 and 2; exponents
+    up to 2^900 for the one-operand forms, 2^60 (the range of a quotient of
+    speeds, densities and pressures in SI units is less) for the others"""
+    rng = np.random.default_rng(11)
+    e = 900 if op in (0, 3) else 60
+    a, b = numbers(rng, 1 << 21, -e, e), numbers(rng, 1 << 21, -e, e)
+    A, B = a.astype(np.longdouble), b.astype(np.longdouble)
+    exact = [1 / A, A / B, A / np.sqrt(B), np.sqrt(A)][op]
+    got = device(lib, op, a, b)
+    assert ulps(got, exact) <= bound, (name, ulps(got, exact))
+    if op == 1:
+        assert np.array_equal(got, a / b)  # corrected by its remainder: the IEEE quotient
+
+
+def test_double_forms_at_the_ends_of_their_ranges(lib):
+    """the smallest and largest operands that still give numbers, and the two
+    roots that are taken of zeros: sqrt0_nb adds 1e-290, fast_speed 1e-280 under
+    its inner root and 1e-290 under the outer one"""
+    a = np.array([1e-307, 1e-300, 1e-200, 1e200, 1e300, 4e307])
+    assert np.allclose(device(lib, 0, a), 1 / a, rtol=2.5e-16, atol=0)
+    assert np.allclose(device(lib, 3, a), np.sqrt(a), rtol=5e-16, atol=0)
+    assert np.allclose(device(lib, 4, [0.0]), 1e-145, rtol=1e-15, atol=0)
+    # fast_speed(gamma p, B^2, 0, 2 rho = 2): sqrt(gamma p + B^2) down to the
+    # clamp, where it is sqrt((G + 1e-140) / 2)
+    gp, b2 = np.array([0.0, 0.0, 1e-100, 1e-30, 1e140]), np.array([0.0, 1e-30, 1e-100, 1e-12, 1e100])
+    assert np.allclose(device(lib, 5, gp, b2), np.sqrt((gp + b2 + np.maximum(gp + b2, 1e-140)) / 2), rtol=1e-15, atol=0)
