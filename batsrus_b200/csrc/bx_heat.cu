@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(512) k_heat_apply(HeatArgs a, const double *__
 // multiply by the pivot reciprocals that the factorisation stores: one
 // double4 or float4 per cell, {lower x, lower y, lower z, 1/pivot}, with zero
 // couplings across block faces and next to unused cells, so that the sweeps
-// need no masks.  The backward sweep reads the same four numbers: the upper
+// need no other masks.  The backward sweep reads the same four numbers: the upper
 // couplings of a cell are the lower ones of its +x, +y, +z neighbours.
 //
 // The factorisation and the sweeps run one warp per block over the 22 planes
@@ -394,6 +394,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) k_heat_factor(HeatArgs a, c
 // the steps.  The block's coefficients and vector lie in shared memory in
 // their natural order: at a step the lanes of a quarter warp have distinct
 // i, so the 16-byte loads of the coefficients are free of bank conflicts.
+// A zero coupling is skipped, not multiplied: what stands in an unused cell
+// (a NaN, an infinity) reaches no other cell.
 //
 // Bytes per cell: coefficients 16 (FP32; FP64 32), r and z 16.  What bounds
 // it is the latency of the 44 steps on small grids and these bytes on large
@@ -454,18 +456,18 @@ __global__ void __launch_bounds__(32 * W) k_heat_ilu(const typename Vec4T<T>::ty
     if ((unsigned)ia < 8u) {
       const V4 v = cf[c0 + ia];
       T s = y[c0 + ia];
-      s = s - v.x * ya;
-      s = s - v.y * pya;
-      s = s - v.z * pza;
+      if (v.x != T(0)) s = s - v.x * ya;
+      if (v.y != T(0)) s = s - v.y * pya;
+      if (v.z != T(0)) s = s - v.z * pza;
       ya = s * v.w;
       y[c0 + ia] = ya;
     }
     if ((unsigned)ib < 8u) {
       const V4 v = cf[c0 + 256 + ib];
       T s = y[c0 + 256 + ib];
-      s = s - v.x * yb;
-      s = s - v.y * pyb;
-      s = s - v.z * pzb;
+      if (v.x != T(0)) s = s - v.x * yb;
+      if (v.y != T(0)) s = s - v.y * pyb;
+      if (v.z != T(0)) s = s - v.z * pzb;
       yb = s * v.w;
       y[c0 + 256 + ib] = yb;
     }
@@ -488,9 +490,9 @@ __global__ void __launch_bounds__(32 * W) k_heat_ilu(const typename Vec4T<T>::ty
       s = s + pza;
       const T zc = y[c0 + ia] - s * v.w;
       y[c0 + ia] = zc;
-      xa = v.x * zc;
-      qa = v.y * zc;
-      ta = v.z * zc;
+      xa = v.x != T(0) ? v.x * zc : T(0);
+      qa = v.y != T(0) ? v.y * zc : T(0);
+      ta = v.z != T(0) ? v.z * zc : T(0);
     }
     if ((unsigned)ib < 8u) {
       const V4 v = cf[c0 + 256 + ib];
@@ -499,9 +501,9 @@ __global__ void __launch_bounds__(32 * W) k_heat_ilu(const typename Vec4T<T>::ty
       if (ka < 3) s = s + pzb;
       const T zc = y[c0 + 256 + ib] - s * v.w;
       y[c0 + 256 + ib] = zc;
-      xb = v.x * zc;
-      qb = v.y * zc;
-      tb = v.z * zc;
+      xb = v.x != T(0) ? v.x * zc : T(0);
+      qb = v.y != T(0) ? v.y * zc : T(0);
+      tb = v.z != T(0) ? v.z * zc : T(0);
     }
   }
   __syncwarp();
