@@ -729,6 +729,7 @@ int gmres(int &iError, cudaStream_t st) {
   if (beta0 == 0.0) return BX_OK;
   double beta = beta0;
   std::vector<double> Hm((m + 1) * m), cs(m), sn(m), g(m + 1), y(m), hb(m + 2);
+  const int steps = kry_gs_steps(kKryAllSteps);
   while (true) {
     k_kry_scale<<<kry_grid(), kKryThreads, 0, st>>>(Vb, H.r, H.scal + 2, 1, N);
     CKH(cudaGetLastError());
@@ -741,7 +742,7 @@ int gmres(int &iError, cudaStream_t st) {
       if ((r = matvec(Vk, H.t, st))) return r;
       if ((r = precond(H.t, H.w, st))) return r;
       if (H.p.TypePrecond == BX_PRECOND_BILU && learned_collecting() && (r = collect_pair(H.t, H.w, st))) return r;
-      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, tune_value(kTuneKryGsSteps), st);  // scal 160..177
+      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, steps, st);  // scal 160..177
       CKH(cudaGetLastError());
       CKH(cudaMemcpyAsync(hb.data(), hdev, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, st));
       CKH(cudaStreamSynchronize(st));
@@ -815,6 +816,7 @@ int fgmres(int &iError, cudaStream_t st) {
   double beta = beta0;
   const double *rvec = H.b;
   std::vector<double> Hm((m + 1) * m), cs(m), sn(m), g(m + 1), y(m), hb(m + 2);
+  const int steps = kry_gs_steps(kKryAllSteps);
   while (true) {
     k_kry_scale<<<kry_grid(), kKryThreads, 0, st>>>(Vb, rvec, H.scal + 2, 1, N);
     CKH(cudaGetLastError());
@@ -826,7 +828,7 @@ int fgmres(int &iError, cudaStream_t st) {
       double *Vk = Vb + (size_t)k * N, *Zk = Zb + (size_t)k * N;
       if ((r = precond(Vk, Zk, st))) return r;
       if ((r = matvec(Zk, H.w, st))) return r;
-      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, tune_value(kTuneKryGsSteps), st);  // scal 160..177
+      kry_orth(H.w, Vb, k, N, hdev, H.scal + 160, H.gram, H.partial, H.cnt, steps, st);  // scal 160..177
       CKH(cudaGetLastError());
       CKH(cudaMemcpyAsync(hb.data(), hdev, sizeof(double) * (k + 2), cudaMemcpyDeviceToHost, st));
       CKH(cudaStreamSynchronize(st));

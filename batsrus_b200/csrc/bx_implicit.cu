@@ -220,7 +220,7 @@ int gmres(int &iError) {
   // three Gram-Schmidt steps per pass unless the caller sets the knob: the
   // finite differences of the products amplify a change of the rounding (the
   // two-pass columns move single cells by up to 1e-6 of the state's norm)
-  const int steps = tune_knob(kTuneKryGsSteps).tuned == 2 ? tune_value(kTuneKryGsSteps) : 3;
+  const int steps = kry_gs_steps(3);
   while (true) {
     k_kry_scale<<<kry_grid(), kKryThreads, 0, c.st>>>(I.V, rvec, I.scal + 2, 1, N);  // V0 = r/||r||
     CKI(cudaGetLastError());

@@ -334,6 +334,8 @@ inline void kry_gs(const GsArgs &a, int na, int nc, cudaStream_t st) {
 // next vector's loads in flight behind the current sums; each warp's two sums
 // of a vector are folded into one butterfly (lane 0 ends with d, lane 1 with G).
 constexpr int kKryAllSteps = 64;  // value of kTuneKryGsSteps
+// the knob's value, or own where it leaves the choice to the solver
+inline int kry_gs_steps(int own) { return tune_value(kTuneKryGsSteps) ? tune_value(kTuneKryGsSteps) : own; }
 constexpr int kKryGramLd = 65;                                  // basis of at most 65 vectors
 constexpr int kKryPieces = 4, kKryTile = kKryThreads * kKryPieces;  // double2 per tile
 constexpr int kKryPartials = 2 * kKryGramLd;                    // sums per CTA

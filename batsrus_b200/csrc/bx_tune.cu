@@ -12,7 +12,7 @@
 
 namespace bx {
 
-static const int g_default[kNumTune] = {4, 4, 2, 1, 192, 0, 64};
+static const int g_default[kNumTune] = {4, 4, 2, 1, 192, 0, 0};
 static TuneKnobInfo g_knobs[kNumTune] = {
     {"stage_ctas_per_sm", 4, {1, 2, 3, 4}, 4, 0, {}},
     {"krylov_ctas_per_sm", 4, {2, 4, 6, 8}, 4, 0, {}},
@@ -23,8 +23,9 @@ static TuneKnobInfo g_knobs[kNumTune] = {
     // 0.60 ms
     {"bilu_threads", 4, {0, 128, 192, 256}, 192, 0, {}},
     {"stage_variant", 4, {0, 1, 2, 3}, 0, 0, {}},
-    // changes the rounding of the Krylov coefficients: a setting, not timed
-    {"krylov_gs_steps", 5, {1, 2, 3, 4, 64}, 64, 0, {}},
+    // changes the rounding of the Krylov coefficients: a setting, not timed;
+    // 0: each solver's own (kry_gs_steps)
+    {"krylov_gs_steps", 6, {0, 1, 2, 3, 4, 64}, 0, 0, {}},
 };
 
 TuneKnobInfo &tune_knob(int knob) { return g_knobs[knob]; }

@@ -14,13 +14,13 @@ enum TuneKnob {
   kTuneStageGrid = 0,  // persistent stage kernel: at most this many CTAs per SM
   kTuneKryCtas,        // Krylov vector kernels: CTAs per SM (256 threads each)
   kTuneKryUnroll,      // Krylov MGS step: independent 16-byte loads in flight per thread and vector
-  kTuneHeatIluWarps,   // heat ILU sweeps: warps (groups of 32 blocks) per CTA
+  kTuneHeatIluWarps,   // heat ILU sweeps: warps (one block each) per CTA
   kTuneBiluThreads,    // JFNK BILU sweeps: threads per block CTA (8 per cell of a wavefront)
   kTuneStageVariant,   // stage kernel, 8^3 blocks: 0 units of 128 cells (bx_stage_unit.cuh); 3 whole blocks
                        // (bx_stage8_launch.cuh); one direction at a time with 1: one face per thread
                        // (576 threads), 2: two (288)
-  kTuneKryGsSteps,     // Gram-Schmidt steps per pass over w (1 to 4, 64: all; implicit step: 3
-                       // unless set); set, not timed
+  kTuneKryGsSteps,     // Gram-Schmidt steps per pass over w (1 to 4, 64: all; 0: each solver's own, all
+                       // for heat conduction, 3 for the implicit step); set, not timed
   kNumTune
 };
 
