@@ -36,3 +36,19 @@ def test_unused_cells_reach_no_other_cell(sweeps, bad):
     assert np.isfinite(z[used]).all()
     assert np.array_equal(y[used], z[used])
     x.close()
+
+
+@pytest.mark.parametrize("sweeps", ["fp64", "fp32"])
+@pytest.mark.parametrize("nRoot", [1, 3])
+def test_any_number_of_warps_gives_the_same_bits(nRoot, sweeps):
+    """1 and 27 blocks: the last CTA of 2 and 4 warps has warps without a block"""
+    x, h, used = system(nRoot, sweeps)
+    r = np.random.default_rng(3).normal(size=h.shape)
+    out = {}
+    for w in capi.tune_info()["heat_ilu_warps"]["candidates"]:
+        capi.tune_set("heat_ilu_warps", w)
+        out[w] = h.precond(r)
+    capi.tune_reset()
+    assert set(out) == {1, 2, 4}
+    assert all(np.array_equal(z, out[1]) for z in out.values())
+    x.close()
