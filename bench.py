@@ -59,6 +59,20 @@ def peaks():
 DRAM_BYTES_PER_CELL_LAUNCH = {"fp64": 169.5, "fp32": 132.0}
 
 
+def stage_variant():
+    """the stage kernel of 8^3 blocks that runs (autotuned or the default)"""
+    from batsrus_b200 import capi
+    return capi.tune_info()["stage_variant"]["value"]
+
+
+def own_launches(flux, variant, steps):
+    """kernels that bx_advance(steps) launches on a uniform grid with graphs off
+    (timing on): two stages per step; the kernel in units (variant 0, not
+    Roe) ends its steps itself and starts a call with one kernel more, the
+    others have two kernels of bookkeeping per step"""
+    return 2 * steps + 1 if variant == 0 and flux != "Roe" else 4 * steps
+
+
 def profile_traffic(prec):
     return DRAM_BYTES_PER_CELL_LAUNCH.get(prec)
 
@@ -188,8 +202,7 @@ def run_ours(args):
                             "unit": "GB/s", "frac": round(achieved / hbm_peak, 4),
                             "traffic": (t_per_cell * nCell if t_per_cell else None),
                             "peak_source": peak_kind},
-               "clocks": clk.summary(), # two stage launches per step and the first step's time step (Roe: two bookkeeping launches more)
-               "gpu_launches": 4 * args.steps if args.flux == "Roe" else 2 * args.steps + 1,
+               "clocks": clk.summary(), "gpu_launches": own_launches(args.flux, stage_variant(), args.steps),
                "autotune": ({k: v["value"] for k, v in tuned.items()} if tuned else None)}
         # ---- end to end through the C ABI with pinned host buffers ----------
         if args.e2e:
