@@ -1,5 +1,5 @@
 // bx_stage.cuh -- block geometry, gather and face states of the per-block
-// kernels (bx_compat.cu).
+// kernels (bx_compat.cu) and of the stage kernel of 2D blocks (bx_stage_flat.cuh).
 #pragma once
 #include <cstdint>
 
@@ -29,10 +29,6 @@ struct Shape {
   static constexpr int NSLOT = 11;  // 8 fluxes, Vdt, BnL, BnR
   __host__ __device__ static constexpr int t(int i, int j, int k) {
     return (i + 2) + TX * ((j + GY) + TY * (k + GZ));
-  }
-  template <typename Real>
-  __host__ __device__ static constexpr size_t smem_bytes() {
-    return sizeof(Real) * (size_t)(8 * NT + NSLOT * NFMAX);
   }
 };
 

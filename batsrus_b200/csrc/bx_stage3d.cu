@@ -12,7 +12,7 @@ namespace bx {
 
 // 8^3 blocks in units or whole (bx_stage8_launch.cuh).  Uniform grids gain by
 // units with Rusanov, Linde and HLLD (160^3 Linde, us per step: FP64 1238 against
-// 1694, FP32-bulk 748 against 789).  With resolution changes the faces of
+// 1694, FP32-bulk 756 against 789).  With resolution changes the faces of
 // their blocks take a long branch, which costs more among the three or four
 // CTAs of an SM than in one set of barriers per block (refined blasts, us per
 // step in units / whole, s the share of blocks at a resolution change):

@@ -8,8 +8,7 @@ namespace {
 
 template <int FLUX>
 cudaError_t launch_flat_flux(const StageArgs &a, cudaStream_t st) {
-  using S = Shape<8, 8, 1>;
-  stage_flat_kernel<S, double, double, double, FLUX><<<a.nBlock, S::NTHREAD, S::template smem_bytes<double>(), st>>>(a);
+  stage_flat_kernel<FLUX><<<a.nBlock, Flat::NTHREAD, 0, st>>>(a);
   return cudaGetLastError();
 }
 

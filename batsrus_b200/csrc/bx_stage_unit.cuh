@@ -25,9 +25,10 @@
 // instructions per cell and stage, 1440 of them FP64 (two cycles each), issue
 // 53 %, FP64 pipe 44 % of the cycles with 15 warps per SM; FP32-bulk 2220
 // instructions, issue 65 %.  Against one CTA per SM and whole blocks
-// (bx_stage3d_v2.cuh): 160^3 per step FP64 Linde 1694 -> 1261 us, HLLD (128^3)
-// 943 -> 692 us, FP32-bulk Linde 789 -> 726 us; 16^3 (8 blocks, now 32 units)
-// 41 -> 23 us; 96^3 cells / 8 in blocks of 4^3 125 -> 57 us.
+// (bx_stage3d_v2.cuh): 160^3 per step FP64 Linde 1694 -> 1238 us, HLLD (128^3)
+// 943 -> 690 us, FP32-bulk Linde 789 -> 756 us; 16^3 (8 blocks, now 32 units)
+// 41 -> 21 us; 96^3 cells / 8 in blocks of 4^3 125 -> 57 us.  With resolution
+// changes: see stage3d_units (bx_stage3d.cu).
 #pragma once
 #include "bx_stage3d.cuh"
 

@@ -1,6 +1,6 @@
 """What ptxas says about the stage kernel of 2D blocks: no flux spills registers
-to local memory.  A limit of registers below what a flux needs (128 for Rusanov,
-148 for Linde, 122 for HLLD and 212 for Roe) costs more than the CTAs that
+to local memory.  A limit of registers below what a flux needs (127 for Rusanov,
+146 for Linde, 116 for HLLD and 206 for Roe) costs more than the CTAs that
 it makes room for."""
 import os
 import re
