@@ -158,32 +158,41 @@ cudaError_t launch_dependent(void (*k)(P...), int grid, int block, size_t smem, 
 // access to the time-step state: the last CTA through ends the time step and
 // sets the next one's, in place of two launches of one thread each (5 us of
 // a step's 23 on a grid of 16^3).  Every CTA has read DtNoCfl and added its
-// minimum before it counts itself.  The steps left and the time limit are
-// read from the state, so that the launches of all steps are alike.
-__device__ __forceinline__ void finish_stage(const StageArgs &a) {
+// minimum before it counts itself.  The steps left and the time limit stand in
+// the state, so that the launches of all steps are alike.  What the last CTA
+// needs but the minimum does not change during the stage: thread 0 of every
+// CTA loads it early (load_step, into shared memory), since a load at the
+// end queues behind the other CTAs' atomics on the same line (two of them
+// cost 2 us of a step at 16^3).
+__device__ __forceinline__ void load_step(const StageArgs &a, StepState &s) {
+  if (!a.finish || threadIdx.x != 0) return;
+  s.DtNoCfl = a.ts->DtNoCfl;
+  s.Dt = a.ts->Dt;
+  s.tSimulation = a.ts->tSimulation;
+  s.nStep = a.ts->nStep;
+  s.nLeft = a.ts->nLeft;
+  s.tLimit = a.ts->tLimit;
+}
+
+__device__ __forceinline__ void finish_stage(const StageArgs &a, const StepState &loaded) {
   if (!a.finish) return;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     if (atomicAdd(&a.ts->nDone, 1u) == gridDim.x - 1) {
       __threadfence();
-      StepState s;
-      s.DtNoCfl = a.ts->DtNoCfl;
-      s.Dt = a.ts->Dt;
-      s.tSimulation = a.ts->tSimulation;
-      s.nStep = a.ts->nStep;
+      StepState s = loaded;
       s.DtMinBits = atomicAdd(&a.ts->DtMinBits, 0ull);
-      const double tLimit = a.ts->tLimit;
-      const int nLeft = a.ts->nLeft - 1;
-      step_end(&s, a.nStage, tLimit);
-      if (nLeft > 0) step_set_dt(&s, tLimit, a.useDtFixed, a.dtFixed, a.cfl);
+      step_end(&s, a.nStage, s.tLimit);
+      s.nLeft = s.nLeft - 1;
+      if (s.nLeft > 0) step_set_dt(&s, s.tLimit, a.useDtFixed, a.dtFixed, a.cfl);
       a.ts->DtNoCfl = s.DtNoCfl;
       a.ts->Dt = s.Dt;
       a.ts->tSimulation = s.tSimulation;
       a.ts->nStep = s.nStep;
       a.ts->DtMinBits = s.DtMinBits;
       a.ts->nDone = 0;
-      a.ts->nLeft = nLeft;
+      a.ts->nLeft = s.nLeft;
     }
   }
 }

@@ -93,6 +93,7 @@ template <int FLUX>
 __global__ void __launch_bounds__(Flat::NTHREAD) stage_flat_kernel(const StageArgs a) {
   using S = Flat;
   __shared__ double tile[8 * S::NT], fbuf[S::NSLOT * S::NFMAX], wmin[S::NTHREAD / 32];
+  __shared__ StepState step;
 
   const int b = a.order[blockIdx.x];
   int nb[6];
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(Flat::NTHREAD) stage_flat_kernel(const StageAr
   const BlockGeom g = a.geom[b];
 
   gather_tile<S, double>(reinterpret_cast<const double *>(a.in), nb, b, tile);
+  load_step(a, step);
   __syncthreads();
 
   CellAcc acc;
@@ -169,7 +171,7 @@ __global__ void __launch_bounds__(Flat::NTHREAD) stage_flat_kernel(const StageAr
       atomicMin(&a.ts->DtMinBits, dbits(m));
     }
   }
-  finish_stage(a);
+  finish_stage(a, step);
 }
 
 }  // namespace bx

@@ -23,6 +23,7 @@ template <class S, int FLUX, int LIM>
 __global__ void __launch_bounds__(S::NTHR, S::MINB) stage_line_kernel(const StageArgs a) {
   constexpr int NI = S::NI, PT = S::PT, NF = S::NF;
   __shared__ double P[8 * PT], fb[11 * NF], wmin[S::NTHR / 32];
+  __shared__ StepState step;
   const int t = threadIdx.x, b = blockIdx.x;  // the owned blocks come first
   const int nb0 = a.nbr[6 * b], nb1 = a.nbr[6 * b + 1];
   const BlockGeom g = a.geom[b];
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(S::NTHR, S::MINB) stage_line_kernel(const Stag
 #pragma unroll
     for (int v = 0; v < 8; v++) o[v] = a.old[(size_t)b * 8 * NI + v * NI + t];
   }
+  load_step(a, step);
   __syncthreads();
 
   if (t < NF) {
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(S::NTHR, S::MINB) stage_line_kernel(const Stag
       atomicMin(&a.ts->DtMinBits, (unsigned long long)__double_as_longlong(m));
     }
   }
-  finish_stage(a);
+  finish_stage(a, step);
 }
 
 }  // namespace bx

@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(W::NTHR, W::MINB)
   __shared__ double wmin[4];
   __shared__ UnitMeta meta[2][NT];
   __shared__ int sTimeout;
+  __shared__ StepState step;
   const int t = threadIdx.x, lane = t & 31, warp = __shfl_sync(0xffffffffu, t >> 5, 0);
   const int nUnit = N == 8 ? 4 * a.nBlock : (a.nBlock + NT - 1) / NT;
   const int nIter = nUnit > (int)blockIdx.x ? (nUnit - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -318,6 +319,7 @@ __global__ void __launch_bounds__(W::NTHR, W::MINB)
   if (t == 0 && nIter > 0) issue_unit<W, TileT>(maps, stg, &bar, meta[0]);
 
   const double DtNoCfl = a.ts->DtNoCfl;
+  load_step(a, step);
   const Real beta = (Real)a.beta, gammaR = (Real)a.gamma, invGm1R = (Real)a.invGm1;
   int err = 0;
   double dtRun = 1e300;  // thread 0: the smallest cell time step of this CTA's units
@@ -566,7 +568,7 @@ __global__ void __launch_bounds__(W::NTHR, W::MINB)
     mbar_wait_bounded(&bar, 0);
     mbar_wait_bounded(&bar, 1);
   }
-  finish_stage(a);
+  finish_stage(a, step);
 }
 
 }  // namespace bx
