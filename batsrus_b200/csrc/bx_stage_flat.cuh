@@ -11,10 +11,11 @@
 // read-only path, so the kernel does not start before the one that writes the
 // state has ended.
 //
-// No limit on the registers: 127 (Rusanov), 146 (Linde), 116 (HLLD) and 206 (Roe)
-// hold five, four, five and three CTAs per SM without spills; a limit of 128
-// for five CTAs spilled 120 bytes of Linde's and 320 of Roe's: Linde 81.2 us
-// per step at 384 x 384 instead of 78.3, 23.0 instead of 21.2 on 10 x 9 blocks.
+// Five CTAs per SM (128 registers), four for Linde (150, no spills): a limit of
+// 128 spills 104 bytes of Linde's (us per step at 384 x 384: 80.6 instead of
+// 78.3, 10 x 9 blocks 22.5 instead of 20.9; 115 instead of 123 at 480 x 480, where
+// five CTAs save a wave).  Rusanov and HLLD fit; Roe spills 320 bytes and gains
+// all the same (210 registers, three CTAs: 181.3 instead of 123.9 us at 384 x 384).
 #pragma once
 #include "bx_stage.cuh"
 
@@ -35,8 +36,7 @@ __device__ __forceinline__ void sweep(const StageArgs &a, const BlockGeom &g, co
                                       CellAcc &acc, int &err) {
   using S = Flat;
   constexpr int NF = D == 0 ? S::NFX : S::NFY;
-  const int f = threadIdx.x;
-  if (f < NF) {
+  for (int f = threadIdx.x; f < NF; f += blockDim.x) {
     int i, j, k;
     face_decode<S, D>(f, i, j, k);
     double L[8], R[8], F[8], vdt;
@@ -90,7 +90,7 @@ __device__ __forceinline__ void sweep(const StageArgs &a, const BlockGeom &g, co
 }
 
 template <int FLUX>
-__global__ void __launch_bounds__(Flat::NTHREAD) stage_flat_kernel(const StageArgs a) {
+__global__ void __launch_bounds__(Flat::NTHREAD, FLUX == kFluxLinde ? 4 : 5) stage_flat_kernel(const StageArgs a) {
   using S = Flat;
   __shared__ double tile[8 * S::NT], fbuf[S::NSLOT * S::NFMAX], wmin[S::NTHREAD / 32];
   __shared__ StepState step;
