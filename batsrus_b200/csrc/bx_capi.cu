@@ -405,7 +405,7 @@ int launch_stage_dt(int iStage, bool computeDt, bool finish = false) {
     }
     e = launch_stage3d(g.shape, g.sch.TypeFlux, kind, *m, a, g.nSM, g.st);
   } else {
-    e = g.shape == kShape881 ? launch_stage_flat(g.sch.TypeFlux, a, g.st)
+    e = g.shape == kShape881 ? launch_stage_flat(g.sch.TypeFlux, a, g.nSM, g.st)
                              : launch_stage_line(g.shape, g.sch.TypeFlux, a, g.st);
   }
   if (e != cudaSuccess) return fail(BX_ERR_CUDA, "stage kernel launch: %s", cudaGetErrorString(e));
@@ -509,8 +509,15 @@ int tune_stage_impl() {
 // The time steps of bx_advance.  Where the stage kernel ends the step itself
 // (StageArgs::finish), a step is its stages: begin_steps sets the first
 // one's time step, and each step sets the next one's while some are left.
-// Elsewhere each step is launched with its own set_dt and end_step kernels.
-bool fused_steps() { return !g.use3d || in_units(); }
+// Elsewhere each step is launched with its own set_dt and end_step kernels:
+// whole 8^3 blocks, and 2D grids of more than three waves of CTAs, where the
+// fence before a CTA counts itself as through costs more than the two launches
+// (us per step with / without, Linde: 90 blocks 20.9 / 22.9, 1024 41.4 / 43.3, 1600
+// 59.8 / 59.8, 2304 78.6 / 76.7).
+bool fused_steps() {
+  if (g.use3d) return in_units();
+  return g.shape != kShape881 || g.nOwned <= 3 * 4 * g.nSM;
+}
 
 int begin_steps(int nStep, double tLimit) {
   begin_steps_kernel<<<1, 1, 0, g.st>>>(g.ts, nStep, tLimit, g.sch.UseDtFixed, g.sch.DtFixed, g.sch.Cfl);
@@ -813,8 +820,8 @@ int bx_init(const bx_grid_desc *gd, const bx_scheme_params *sp) {
   g.bufX = g.A;
   g.bufY = g.B;
   g.use3d = g.shape == kShape888 || g.shape == kShape444;
+  CK(cudaDeviceGetAttribute(&g.nSM, cudaDevAttrMultiProcessorCount, g.dev));
   if (g.use3d) {
-    CK(cudaDeviceGetAttribute(&g.nSM, cudaDevAttrMultiProcessorCount, g.dev));
     r = encode_maps(g.bufX, false, g.nI, g.nBlock, g.mapX64);
     if (!r) r = encode_maps(g.bufY, false, g.nI, g.nBlock, g.mapY64);
     if (!r) r = encode_maps(g.bufY, true, g.nI, g.nBlock, g.mapY32);

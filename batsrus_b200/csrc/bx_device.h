@@ -224,7 +224,7 @@ enum { kShape888 = 0, kShape444 = 1, kShape881 = 2, kShape811 = 3, kShape6411 = 
 // launchers (explicitly instantiated in bx_stage_line.cu, bx_stage_flat.cu and
 // bx_compat.cu): 1D blocks, 2D blocks
 cudaError_t launch_stage_line(int shape, int flux, const StageArgs &a, cudaStream_t st);
-cudaError_t launch_stage_flat(int flux, const StageArgs &a, cudaStream_t st);
+cudaError_t launch_stage_flat(int flux, const StageArgs &a, int nSM, cudaStream_t st);
 cudaError_t launch_compat(int shape, int flux, int phase, int iBlock, const CompatArgs &a,
                           cudaStream_t st);
 // persistent TMA-staged kernel of 3D shapes (bx_stage3d.cu): tensor maps of

@@ -11,11 +11,12 @@
 // read-only path, so the kernel does not start before the one that writes the
 // state has ended.
 //
-// Five CTAs per SM (128 registers), four for Linde (150, no spills): a limit of
-// 128 spills 104 bytes of Linde's (us per step at 384 x 384: 80.6 instead of
-// 78.3, 10 x 9 blocks 22.5 instead of 20.9; 115 instead of 123 at 480 x 480, where
-// five CTAs save a wave).  Rusanov and HLLD fit; Roe spills 320 bytes and gains
-// all the same (210 registers, three CTAs: 181.3 instead of 123.9 us at 384 x 384).
+// Five CTAs per SM (128 registers): Rusanov and HLLD fit; Roe spills 320 bytes
+// and gains all the same (210 registers, three CTAs: 181 instead of 124 us per
+// step at 384 x 384).  Linde needs 150 registers, for four; with the limit of 128
+// it spills 104 bytes.  It takes five where that saves a wave of CTAs, else four
+// (us per step with four / five: 90 blocks 20.9 / 22.5, 1024 41.4 / 43.5, 1600
+// 59.8 / 61.6, 2304 78.6 / 80.6, but 1357 blocks 54 / 46, 3600 123 / 115).
 #pragma once
 #include "bx_stage.cuh"
 
@@ -89,8 +90,9 @@ __device__ __forceinline__ void sweep(const StageArgs &a, const BlockGeom &g, co
   __syncthreads();
 }
 
-template <int FLUX>
-__global__ void __launch_bounds__(Flat::NTHREAD, FLUX == kFluxLinde ? 4 : 5) stage_flat_kernel(const StageArgs a) {
+// CTAS: CTAs per SM that the register limit allows for
+template <int FLUX, int CTAS>
+__global__ void __launch_bounds__(Flat::NTHREAD, CTAS) stage_flat_kernel(const StageArgs a) {
   using S = Flat;
   __shared__ double tile[8 * S::NT], fbuf[S::NSLOT * S::NFMAX], wmin[S::NTHREAD / 32];
   __shared__ StepState step;

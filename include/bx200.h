@@ -465,8 +465,9 @@ BX_API int bx_heat_precond(const double *r, double *z);
  * ILU after bx_heat_init, the BILU sweeps after an implicit BILU step, the
  * Krylov vector kernels always) with CUDA events on the live data and keeps
  * the fastest.  Knobs set by bx_tune_set are kept.  The candidates of a knob
- * compute the same result, except the Krylov grid, which sets the summation
- * order of the GMRES inner products. */
+ * compute the same result, but for the rounding of the Krylov grid, which sets
+ * the summation order of the GMRES inner products, and of the stage kernel's
+ * variant. */
 BX_API int bx_autotune(void);
 /* knob iKnob (0-based; BX_ERR_ARG past the last): name (nameLen bytes),
  * current value, tuned (0 default, 1 autotuned, 2 set by the caller), the

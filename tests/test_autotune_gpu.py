@@ -42,8 +42,9 @@ def test_stage_grid_candidates_bit_identical():
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_stage_variants_agree(prec):
-    """The three 8^3 stage kernels (one face phase; one direction at a time
-    with one or two faces per thread) on a blast state with HLLD and Linde
+    """The 8^3 stage kernels (units of 128 cells or whole blocks by the grid; whole
+    blocks; one direction at a time with one or two faces per thread) on a
+    blast state with HLLD and Linde
     and the Koren limiter, on a static AMR grid with resolution changes, and
     in the implicit residual mode: the same state to rounding."""
     out = {}
@@ -82,7 +83,7 @@ def heat_case(nRoot=2, prec="BILU"):
 
 
 def test_heat_ilu_warps_bit_identical():
-    x, h, _ = heat_case(nRoot=4)  # 512 blocks: 16 groups of 32
+    x, h, _ = heat_case(nRoot=4)  # 64 blocks: full CTAs with 1, 2 and 4 warps (others: test_heat_sweeps_gpu.py)
     r = np.random.default_rng(3).normal(size=h.shape)
     out = {}
     for w in capi.tune_info()["heat_ilu_warps"]["candidates"]:

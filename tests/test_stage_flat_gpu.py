@@ -1,5 +1,5 @@
-"""The stage kernel of 1D and 2D blocks (one thread per face, the end of the
-time step inside the last stage) against the oracle: every block shape, one
+"""The stage kernels of 1D blocks (one thread per face) and of 2D blocks (one
+sweep per direction), which end the time step in the last stage, against the oracle: every block shape, one
 block (its own periodic neighbour), odd counts, float sides, both orders, and
 step counts that end a call right after one, two and several graph replays,
 with a time limit in the last step.  A step's rounding is a few 1e-16; 1e-12
